@@ -228,7 +228,7 @@ def build_adapter(cpu_objs: list[str], flags: list[str]) -> None:
 
 
 def main() -> int:
-    if not REF.is_dir():
+    if not (REF / "kpz").is_dir():
         print(f"{REF} not present; skipping the reference build", file=sys.stderr)
         return 0
     if WORK.exists():
