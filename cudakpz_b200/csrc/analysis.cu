@@ -4,15 +4,15 @@
 // Heights follow the reference's path walk (kpz/correlator.cpp:47-96, :337-399):
 //   row y starts at Hs(y) = h(0,y-1) + (2*s_y(0,y)-1) with h(0,-1) = 0, walks x = 1..L-1
 //   adding 2*s_x(x,y)-1, and the wrap adds 2*s_x(0,y)-1 giving h(0,y) = Hs(y) + rowsum(y).
-// Moments: S1 and S2 exact in int64, S3..S7 in FP64 (per 64-site chunk from exact integer
-// power sums of the offsets from the chunk's first height); ch uses the exact int64 cross sum;
-// cs counts equal minus different slope bits (kpz/correlator.cpp:463-477).
+// Moments: S1 and S2 exact in int64, S3..S7 in FP64 from exact integer counts (below); ch uses
+// the exact int64 cross sum; cs counts equal minus different slope bits
+// (kpz/correlator.cpp:463-477).
 // Invariants extend SchedulerService::consitencyCheck (kpz/schedulerService.cpp:733-854)
 // to ENC_CBBIT: x-slope row sums, y-slope column sums, plaquette loops.
 //
-// Three passes: (1) per-row x=0 slopes and x-slope sums, (2) one-CTA scan over rows to
-// get row-start heights, (3) per-site walk with a CTA-wide scan of 64-site chunk sums.
-// Per-CTA partials are reduced in a fixed order so the FP64 sums are deterministic.
+// Two launches: (1) row_kernel: per-row slope counts and the row starts within a block of rows;
+// (2) walk_kernel: the walk in groups of eight sites from the block totals on, whose last CTA adds
+// the per-CTA partials in a fixed order, so the FP64 sums are deterministic.
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -22,8 +22,12 @@
 
 namespace kpzb {
 
-constexpr int AN_THREADS = 256;
-constexpr int AN_MAX_GRID = 1184;
+constexpr int AN_MAX_GRID = 148;  // CTAs of the walk: one per SM of a B200
+constexpr int AN_ROW_THREADS = 256;
+// Lattices of at least 128 words per quadrant row are walked in four parts per row, each by its
+// own warp: 16384^2 is then 13.8 parts per warp instead of 3.5 rows (a last wave 1.3 % short
+// instead of 14 %).
+constexpr int AN_PART_WORDS = 128;
 
 struct Partial {
     long long s1, s2, hmin, hmax, cross, agree, snap_s1, pad;
@@ -31,303 +35,608 @@ struct Partial {
     double pad2[3];
 };
 
-// ---- pass 1: per-row x=0 slopes and x-slope row sums (one warp per row) ----
-__global__ void rowinfo_kernel(const uint32_t* __restrict__ sys, int lx, int ly, int32_t* rowinfo)
-{
-    const uint64_t Wr = 1ull << (lx - 6);
-    const uint64_t Q = 1ull << (lx + ly - 6);
-    const uint64_t rows = 1ull << ly;
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t y = warp; y < rows; y += nwarps) {
-        int cnt = 0;
-        for (uint64_t j = lane; j < Wr; j += 32)
-            cnt += __popc(sys[y * Wr + j]) + __popc(sys[2 * Q + y * Wr + j]);
-        for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        if (lane == 0) {
-            // site (0,y) lies on sublattice y&1, word 0, bit 0
-            const uint64_t b0 = (y & 1) ? 2 * Q : 0;
-            const int sy0 = (int)(sys[b0 + Q + y * Wr] & 1u);
-            rowinfo[2 * y] = 2 * sy0 - 1;
-            rowinfo[2 * y + 1] = 2 * cnt - (int)(1ull << lx);
-        }
-    }
-}
+// Per-row record {n1, n2, n3, w}: the X-slope bits set in the row's first one, two and three
+// quarters (rows of at least AN_PART_WORDS words; else 0), and w = x-slope row sum (even) with the
+// y-slope bit of x = 0 in bit 0.
+__device__ __forceinline__ int row_sum(int w) { return w & ~1; }
+__device__ __forceinline__ int row_ystep(int w) { return 2 * (w & 1) - 1; }
 
-// ---- pass 2: row-start heights Hs(y) (single CTA, chunked Hillis-Steele scan) ----
-__global__ void rowstart_kernel(const int32_t* __restrict__ rowinfo, int ly, int64_t* rowstart)
-{
-    __shared__ long long buf[1024];
-    __shared__ long long carry;
-    const uint64_t rows = 1ull << ly;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (uint64_t base = 0; base < rows; base += 1024) {
-        const uint64_t y = base + threadIdx.x;
-        // Hs(y) = sum_{y'<=y} ycol(y') + sum_{y'<y} rowsum(y')
-        // contribution of row y to the inclusive scan: ycol(y) + rowsum(y-1) handled as
-        // v(y) = ycol(y) + rowsum(y); Hs(y) = incl(v)(y) - rowsum(y)
-        long long v = (y < rows) ? (long long)rowinfo[2 * y] + rowinfo[2 * y + 1] : 0;
-        buf[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            long long add = (threadIdx.x >= (unsigned)o) ? buf[threadIdx.x - o] : 0;
-            __syncthreads();
-            buf[threadIdx.x] += add;
-            __syncthreads();
-        }
-        if (y < rows) rowstart[y] = carry + buf[threadIdx.x] - rowinfo[2 * y + 1];
-        __syncthreads();
-        if (threadIdx.x == 1023) carry += buf[1023];
-        __syncthreads();
-    }
-}
+// Rows are scanned in up to AN_MAX_BLOCKS blocks of 2^lgb rows: rowstart[y] is relative to the
+// start of y's block, and the block's record holds its total step and the extremes of its starts.
+constexpr int AN_MAX_BLOCKS = 256;
+struct RowBlock {
+    long long total, lo, hi;
+};
+__host__ __device__ constexpr int row_block_lg(int ly) { return ly <= 12 ? (ly < 4 ? ly : 4) : ly - 8; }
 
-// ---- pass 3: per-site walk ----
-// MODE 0: moments; MODE 1: moments + correlate against snap; MODE 2: write heights.
-template <int MODE>
-__global__ void __launch_bounds__(AN_THREADS)
-walk_kernel(const uint32_t* __restrict__ sys, const uint32_t* __restrict__ snap, int lx, int ly,
-            const int32_t* __restrict__ rowinfo, const int64_t* __restrict__ rowstart,
-            const int32_t* __restrict__ rowinfo_s, const int64_t* __restrict__ rowstart_s,
-            int32_t* __restrict__ heights, Partial* __restrict__ partials)
-{
-    __shared__ long long wsum[AN_THREADS / 32];
-    __shared__ long long wsum_s[AN_THREADS / 32];
-    __shared__ long long segc[AN_THREADS];
-    __shared__ long long segc_s[AN_THREADS];
+// What the kernels leave in the scratch beside the partial sums: the row blocks of the system and
+// of the snapshot, and the walk's last-CTA ticket (cleared by every row_kernel, so a count left
+// over by callers that raced on a shared scratch does not outlive the next call).
+struct WalkState {
+    RowBlock block[2][AN_MAX_BLOCKS];
+    unsigned int ticket;
+};
 
-    const uint64_t Wr = 1ull << (lx - 6);
-    const uint64_t Q = 1ull << (lx + ly - 6);
-    const uint64_t rows = 1ull << ly;
-    const int TPR = (int)(Wr < AN_THREADS ? Wr : AN_THREADS);
-    const int RPC = AN_THREADS / TPR;
-    const int tx = threadIdx.x % TPR, ty = threadIdx.x / TPR;
+// Exclusive scan of one int64 per thread over a CTA of NT threads; *total = the sum.
+template <int NT>
+__device__ __forceinline__ long long cta_exclusive_scan(long long v, long long* total)
+{
+    __shared__ long long wsum[NT / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int nseg = (int)(Wr / TPR);
-    const uint64_t groups = rows / RPC;
-    const uint64_t L = 1ull << lx;
-
-    long long s1 = 0, s2 = 0, cross = 0, agree = 0, ss1 = 0;
-    long long hmin = 0x7fffffffffffffffll, hmax = -0x7fffffffffffffffll;
-    double s3 = 0, s4 = 0, s5 = 0, s6 = 0, s7 = 0;
-
-    for (uint64_t g = blockIdx.x; g < groups; g += gridDim.x) {
-        const uint64_t y = g * RPC + ty;
-        const uint64_t be = (y & 1) ? 2 * Q : 0, bo = (y & 1) ? 0 : 2 * Q;
-        const long long Hs = rowstart[y];
-        const long long rsum = rowinfo[2 * y + 1];
-        long long Hs_s = 0, rsum_s = 0;
-        if (MODE == 1) {
-            Hs_s = rowstart_s[y];
-            rsum_s = rowinfo_s[2 * y + 1];
-        }
-        // e0 = 2*s_x(0,y)-1 (bit 0 of the even-x word 0)
-        const long long e0 = 2 * (long long)(sys[be + y * Wr] & 1u) - 1;
-        long long e0_s = 0;
-        if (MODE == 1) e0_s = 2 * (long long)(snap[be + y * Wr] & 1u) - 1;
-        long long run = 0, run_s = 0;  // prefix carried from previous segments
-        for (int seg = 0; seg < nseg; ++seg) {
-            const uint64_t c = (uint64_t)seg * TPR + tx;
-            const uint32_t E = sys[be + y * Wr + c], O = sys[bo + y * Wr + c];
-            uint32_t Es = 0, Os = 0;
-            if (MODE == 1) {
-                Es = snap[be + y * Wr + c];
-                Os = snap[bo + y * Wr + c];
-                const uint32_t EY = sys[be + Q + y * Wr + c], OY = sys[bo + Q + y * Wr + c];
-                const uint32_t EYs = snap[be + Q + y * Wr + c], OYs = snap[bo + Q + y * Wr + c];
-                agree += 2 * (__popc(~(E ^ Es)) + __popc(~(O ^ Os)) + __popc(~(EY ^ EYs)) +
-                              __popc(~(OY ^ OYs))) - 128;
-            }
-            long long v = 2 * (__popc(E) + __popc(O)) - 64;
-            long long vs = (MODE == 1) ? 2 * (__popc(Es) + __popc(Os)) - 64 : 0;
-            // inclusive scan of v over the TPR threads of this row
-            long long incl = v, incl_s = vs;
-            const int wl = TPR < 32 ? TPR : 32;
-            for (int o = 1; o < wl; o <<= 1) {
-                long long a = __shfl_up_sync(0xffffffffu, incl, o, wl);
-                long long as = __shfl_up_sync(0xffffffffu, incl_s, o, wl);
-                if ((lane % wl) >= o) {
-                    incl += a;
-                    incl_s += as;
-                }
-            }
-            if (TPR > 32) {
-                if (lane == 31) {
-                    wsum[wid] = incl;
-                    wsum_s[wid] = incl_s;
-                }
-                __syncthreads();
-                const int w0 = (ty * TPR) >> 5;  // first warp of this row
-                for (int w = w0; w < wid; ++w) {
-                    incl += wsum[w];
-                    incl_s += wsum_s[w];
-                }
-            }
-            // P(x) before this chunk (inclusive prefix from x = 0)
-            long long P = run + incl - v;
-            long long Ps = run_s + incl_s - vs;
-            // last thread of the row publishes the segment total
-            if (tx == TPR - 1) {
-                segc[ty] = run + incl;
-                segc_s[ty] = run_s + incl_s;
-            }
-            __syncthreads();
-            run = segc[ty];
-            run_s = segc_s[ty];
-            __syncthreads();
-            if constexpr (MODE == 0) {
-                // The chunk's heights are b + d_i with b the height before its first site and
-                // |d_i| <= 64, so the power sums of d are exact in 32/64-bit integers (d^4 sums to
-                // at most 64 * 64^4 < 2^31; d^5..d^7 accumulate in int64) and the moments of h
-                // follow once per chunk by the binomial expansion in FP64.  The row's first site
-                // (x = 0, height Hs + rowsum) is left out of the sums and added directly.
-                const long long b = Hs - e0 + P;
-                const bool first = c == 0;
-                int d = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0, dmin = 64, dmax = -64;
-                long long a5 = 0, a6 = 0, a7 = 0;
+    long long incl = v;
 #pragma unroll
-                for (int i = 0; i < 64; ++i) {
-                    const int bit = (int)((((i & 1) ? O : E) >> (i >> 1)) & 1u);
-                    d += 2 * bit - 1;
-                    if (i == 0 && first) continue;
-                    const int d2 = d * d, d3 = d2 * d, d4 = d2 * d2;
-                    a1 += d;
-                    a2 += d2;
-                    a3 += d3;
-                    a4 += d4;
-                    a5 += (long long)d4 * d;
-                    a6 += (long long)d3 * d3;
-                    a7 += (long long)d4 * d3;
-                    dmin = min(dmin, d);
-                    dmax = max(dmax, d);
-                }
-                const int n = first ? 63 : 64;
-                s1 += (long long)n * b + a1;
-                s2 += (long long)n * b * b + 2 * b * a1 + a2;
-                hmin = min(hmin, b + dmin);
-                hmax = max(hmax, b + dmax);
-                const double B = (double)b, B2 = B * B, B3 = B2 * B, B4 = B2 * B2, B5 = B4 * B, B6 = B3 * B3,
-                             B7 = B6 * B;
-                const double n_ = n, A1 = a1, A2 = a2, A3 = a3, A4 = a4, A5 = (double)a5, A6 = (double)a6,
-                             A7 = (double)a7;
-                s3 += n_ * B3 + 3.0 * B2 * A1 + 3.0 * B * A2 + A3;
-                s4 += n_ * B4 + 4.0 * B3 * A1 + 6.0 * B2 * A2 + 4.0 * B * A3 + A4;
-                s5 += n_ * B5 + 5.0 * B4 * A1 + 10.0 * B3 * A2 + 10.0 * B2 * A3 + 5.0 * B * A4 + A5;
-                s6 += n_ * B6 + 6.0 * B5 * A1 + 15.0 * B4 * A2 + 20.0 * B3 * A3 + 15.0 * B2 * A4 + 6.0 * B * A5 + A6;
-                s7 += n_ * B7 + 7.0 * B6 * A1 + 21.0 * B5 * A2 + 35.0 * B4 * A3 + 35.0 * B3 * A4 + 21.0 * B2 * A5 +
-                      7.0 * B * A6 + A7;
-                if (first) {
-                    const long long h = Hs + rsum;
-                    s1 += h;
-                    s2 += h * h;
-                    const double dh = (double)h, dh2 = dh * dh, dh3 = dh2 * dh;
-                    s3 += dh3;
-                    s4 += dh2 * dh2;
-                    s5 += dh3 * dh2;
-                    s6 += dh3 * dh3;
-                    s7 += dh3 * dh3 * dh;
-                    hmin = min(hmin, h);
-                    hmax = max(hmax, h);
-                }
-                continue;
-            }
-            for (int i = 0; i < 64; ++i) {
-                const uint32_t bit = (((i & 1) ? O : E) >> (i >> 1)) & 1u;
-                P += 2 * (long long)bit - 1;
-                const uint64_t x = c * 64 + i;
-                const long long h = (x == 0) ? Hs + rsum : Hs - e0 + P;
-                if (MODE == 2) {
-                    heights[y * L + x] = (int32_t)h;
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long a = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += a;
+    }
+    if (lane == 31) wsum[wid] = incl;
+    __syncthreads();
+    long long before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+        const long long s = wsum[w];
+        if (w < wid) before += s;
+        all += s;
+    }
+    __syncthreads();
+    *total = all;
+    return before + incl - v;
+}
+
+// ---- launch 1: per-row slope counts and row starts within a block of rows ----
+// A CTA takes one block of rows; blockIdx.y picks the lattice (the system, the snapshot).  A warp
+// reads a row's 2 Wr words as 128-bit loads, ordered quarter by quarter and both X quadrants of
+// a quarter together, so that every lane has a load of every step; rows shorter than
+// AN_PART_WORDS take Wr / 2 lanes each.  The scan over blocks is left to each reader, which needs
+// no grid-wide step: a scan of all rows by one CTA (a launch of its own, or the last CTA here)
+// took 15 to 27 us at 8192 and 16384 rows, most of both kernels' time.
+__global__ void __launch_bounds__(AN_ROW_THREADS)
+row_kernel(const uint32_t* __restrict__ sys0, const uint32_t* __restrict__ sys1, int lx, int ly,
+           int4* __restrict__ rowinfo0, int64_t* __restrict__ rowstart0, WalkState* ws)
+{
+    __shared__ int w_s[AN_ROW_THREADS];
+    __shared__ long long lo_s[AN_ROW_THREADS / 32], hi_s[AN_ROW_THREADS / 32];
+    const uint64_t Wr = 1ull << (lx - 6);
+    const uint64_t Q = 1ull << (lx + ly - 6);
+    const uint64_t rows = 1ull << ly;
+    const uint32_t* sys = blockIdx.y ? sys1 : sys0;
+    int4* rowinfo = rowinfo0 + blockIdx.y * rows;
+    int64_t* rowstart = rowstart0 + blockIdx.y * rows;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr int NWARP = AN_ROW_THREADS / 32;
+    const int lgb = row_block_lg(ly);
+    const uint64_t yb = (uint64_t)blockIdx.x << lgb, ye = yb + (1ull << lgb);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) ws->ticket = 0u;
+    auto count4 = [](uint4 v) { return __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w); };
+    // site (0,y) lies on sublattice y&1, word 0, bit 0
+    auto sy0 = [&](uint64_t y) { return (int)(sys[((y & 1) ? 2 * Q : 0) + Q + y * Wr] & 1u); };
+    long long carry = 0, lo = 0x7fffffffffffffffll, hi = -0x7fffffffffffffffll;
+    for (uint64_t base = yb; base < ye; base += AN_ROW_THREADS) {
+        const uint64_t end = ye - base < AN_ROW_THREADS ? ye : base + AN_ROW_THREADS;
+        auto put = [&](uint64_t y, int n1, int n2, int n3, int n, int s) {
+            const int w = (int)(2 * (int64_t)n - (int64_t)(1ull << lx)) | s;
+            rowinfo[y] = make_int4(n1, n2, n3, w);
+            w_s[y - base] = w;
+        };
+        if (Wr >= AN_PART_WORDS) {
+            const uint64_t qv = Wr / 16;  // 128-bit loads per quadrant row quarter (at least 8)
+#pragma unroll 2
+            for (uint64_t y = base + wid; y < end; y += NWARP) {
+                const int s = sy0(y);
+                const uint4* r0 = reinterpret_cast<const uint4*>(sys + y * Wr);
+                const uint4* r1 = reinterpret_cast<const uint4*>(sys + 2 * Q + y * Wr);
+                int n[4] = {0, 0, 0, 0};
+                if (qv == 8) {  // a step of the warp covers two quarters
+                    uint4 v[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) v[h] = (lane & 8 ? r1 : r0)[16 * h + 8 * (lane >> 4) + (lane & 7)];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int c = count4(v[h]);
+                        n[2 * h] = lane < 16 ? c : 0;
+                        n[2 * h + 1] = lane < 16 ? 0 : c;
+                    }
                 } else {
-                    s1 += h;
-                    s2 += h * h;
-                    const double d = (double)h, d2 = d * d, d3 = d2 * d;
-                    s3 += d3;
-                    s4 += d2 * d2;
-                    s5 += d3 * d2;
-                    s6 += d3 * d3;
-                    s7 += d3 * d3 * d;
-                    hmin = min(hmin, h);
-                    hmax = max(hmax, h);
-                    if (MODE == 1) {
-                        const uint32_t bs = (((i & 1) ? Os : Es) >> (i >> 1)) & 1u;
-                        Ps += 2 * (long long)bs - 1;
-                        const long long hs = (x == 0) ? Hs_s + rsum_s : Hs_s - e0_s + Ps;
-                        cross += h * hs;
-                        ss1 += hs;
+                    for (uint64_t i = lane; i < 2 * qv; i += 32) {
+                        uint4 v[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) v[q] = i >= qv ? r1[q * qv + i - qv] : r0[q * qv + i];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) n[q] += count4(v[q]);
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) n[q] = __reduce_add_sync(0xffffffffu, n[q]);
+                if (lane == 0) put(y, n[0], n[0] + n[1], n[0] + n[1] + n[2], n[0] + n[1] + n[2] + n[3], s);
+            }
+        } else {
+            const int sw = (int)(Wr / 2), rpw = 32 / sw;  // lanes per row, rows per warp (powers of two)
+            for (uint64_t y0 = base + (uint64_t)wid * rpw; y0 < end; y0 += (uint64_t)NWARP * rpw) {
+                const uint64_t y = y0 + lane / sw;
+                const int j = lane % sw, half = sw / 2;
+                const bool in = y < end;
+                const int s = in ? sy0(y) : 0;
+                int n = in ? count4(reinterpret_cast<const uint4*>(sys + (j >= half ? 2 * Q : 0) + y * Wr)[j % half]) : 0;
+                for (int o = 1; o < sw; o <<= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+                if (in && j == 0) put(y, 0, 0, 0, n, s);
+            }
+        }
+        if (!rowstart0) continue;  // counts only
+        __syncthreads();
+        // Hs(y) = sum_{y'<=y} ystep(y') + sum_{y'<y} rowsum(y')
+        const uint64_t y = base + threadIdx.x;
+        const int w = y < end ? w_s[threadIdx.x] : 0;
+        const long long v = y < end ? row_ystep(w) + row_sum(w) : 0;
+        long long total;
+        const long long start = carry + cta_exclusive_scan<AN_ROW_THREADS>(v, &total) + row_ystep(w);
+        if (y < end) {
+            rowstart[y] = start;
+            lo = min(lo, start);
+            hi = max(hi, start);
+        }
+        carry += total;
+    }
+    if (!rowstart0) return;
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) {
+        lo_s[wid] = lo;
+        hi_s[wid] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < NWARP; ++w) {
+            lo = min(lo, lo_s[w]);
+            hi = max(hi, hi_s[w]);
+        }
+        ws->block[blockIdx.y][blockIdx.x] = RowBlock{carry, lo, hi};
+    }
+}
+
+// Heights at the start of every row block into base_s (an array of AN_MAX_BLOCKS in shared
+// memory) and the middle of the row starts; NT >= AN_MAX_BLOCKS threads, all of them.
+template <int NT>
+__device__ __forceinline__ long long row_block_bases(const RowBlock* blocks, int nblk, long long* base_s)
+{
+    __shared__ long long lo_s[NT / 32], hi_s[NT / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    RowBlock b{0, 0x7fffffffffffffffll, -0x7fffffffffffffffll};
+    const bool in = (int)threadIdx.x < nblk;
+    if (in) b = blocks[threadIdx.x];
+    long long total;
+    const long long base = cta_exclusive_scan<NT>(b.total, &total);
+    if (in) {
+        base_s[threadIdx.x] = base;
+        b.lo += base;
+        b.hi += base;
+    }
+    if (wid < AN_MAX_BLOCKS / 32)
+        for (int o = 16; o > 0; o >>= 1) {
+            b.lo = min(b.lo, __shfl_xor_sync(0xffffffffu, b.lo, o));
+            b.hi = max(b.hi, __shfl_xor_sync(0xffffffffu, b.hi, o));
+        }
+    if (lane == 0) {
+        lo_s[wid] = b.lo;
+        hi_s[wid] = b.hi;
+    }
+    __syncthreads();
+    long long lo = lo_s[0], hi = hi_s[0];
+#pragma unroll
+    for (int w = 1; w < AN_MAX_BLOCKS / 32; ++w) {
+        lo = min(lo, lo_s[w]);
+        hi = max(hi, hi_s[w]);
+    }
+    __syncthreads();
+    return (lo + hi) >> 1;
+}
+
+// ---- launch 2: the walk ----
+//
+// A group of eight sites is its height H before the first site and an 8-bit slope pattern, so
+// the sums of h^k over the lattice follow from counts of (H, pattern) alone.  Each CTA keeps the
+// counts of WALK_BINS heights of one parity x 256 patterns in shared memory and adds one per
+// group: a shared atomic and about ten integer instructions for eight sites, where evaluating
+// the powers site by site took about 17 instructions a site (330 us against 49 us at 2^28 sites,
+// where the integer ALU bound it; now the shared atomics do; 70 against 25 us at 2^26).  The even rows' groups all have
+// heights of one parity and the odd rows' of the other, so a CTA walks rows of one parity and
+// a bin covers two heights.  At the end thread (pattern p, slice of heights) takes the power
+// sums of H over its bins and combines them with the pattern's own offsets' power sums.
+//
+// Counts are exact and the bins' heights span less than 2^9, so every term up to k = 7 of a
+// surface with |H| <= 16 is an exact integer in FP64; above that the terms of one bin do not
+// cancel (offsets within a group are at most 8).
+//
+// The bins cover WALK_REACH heights on each side of the middle of the row starts (a surface of
+// 16384^2 has heights within about 30 of its mean at t = 10^4).  A chunk of 64 sites that leaves
+// them is summed site by site, as is a row's first chunk when the row's slopes do not close.
+constexpr int WALK_BINS = 192;
+constexpr int WALK_REACH = WALK_BINS - 64;  // a chunk moves at most 64 from its first height
+constexpr int WALK_LUT = 256;
+constexpr int WALK_SMEM = WALK_BINS * 256 * 4;
+
+// Number of set bits of each byte.
+__device__ __forceinline__ uint32_t byte_popc(uint32_t v)
+{
+    v -= (v >> 1) & 0x55555555u;
+    v = (v & 0x33333333u) + ((v >> 2) & 0x33333333u);
+    return (v + (v >> 4)) & 0x0F0F0F0Fu;
+}
+
+struct Sums {
+    long long s1, s2, hmin, hmax;
+    double s[5];
+    __device__ void add_height(long long h)
+    {
+        s1 += h;
+        s2 += h * h;
+        const double d = (double)h, d2 = d * d, d3 = d2 * d;
+        s[0] += d3;
+        s[1] += d2 * d2;
+        s[2] += d3 * d2;
+        s[3] += d3 * d3;
+        s[4] += d3 * d3 * d;
+        hmin = min(hmin, h);
+        hmax = max(hmax, h);
+    }
+};
+
+// One word of a Partial: its value over the CTA's threads, by the warp that reads it.  Words 0, 1
+// and 4-6 are added as integers, 2 and 3 are the extremes, the rest are added in FP64.
+constexpr int PARTIAL_SUMS = 12;
+__device__ __forceinline__ int partial_word(int q) { return q < 7 ? q : q + 1; }
+
+// Reduce a Partial per thread to *out: every thread stores its twelve values to buf (in shared
+// memory, 12 * NT words) and a warp adds up each quantity, lane by lane and then by a tree, in the
+// same order in every call.  (Shuffling all twelve 64-bit values through every warp took 4 us.)
+template <int NT>
+__device__ __forceinline__ void cta_partial(const Partial& p, long long* buf, Partial* out)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long* pw = reinterpret_cast<const long long*>(&p);
+#pragma unroll
+    for (int q = 0; q < PARTIAL_SUMS; ++q) buf[q * NT + threadIdx.x] = pw[partial_word(q)];
+    __syncthreads();
+    if (wid < PARTIAL_SUMS) {
+        const long long* v = buf + wid * NT + lane;
+        long long* o = reinterpret_cast<long long*>(out) + partial_word(wid);
+        if (wid >= 7) {
+            double s = 0.0;
+            for (int i = 0; i < NT; i += 32) s += __longlong_as_double(v[i]);
+            for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+            if (lane == 0) *o = __double_as_longlong(s);
+        } else {
+            const bool lo = wid == 2, hi = wid == 3;
+            long long s = v[0];
+            auto merge = [&](long long x) { s = lo ? min(s, x) : hi ? max(s, x) : s + x; };
+            for (int i = 32; i < NT; i += 32) merge(v[i]);
+            for (int k = 16; k > 0; k >>= 1) merge(__shfl_xor_sync(0xffffffffu, s, k));
+            if (lane == 0) *o = s;
+        }
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ Partial empty_partial()
+{
+    Partial p{};
+    p.hmin = 0x7fffffffffffffffll;
+    p.hmax = -0x7fffffffffffffffll;
+    return p;
+}
+
+// CORR: also the correlator's sums against `snap` (cross sum of heights, agreeing slopes).  Its
+// heights relative to the two lattices' middles are built as biased bytes from a table of
+// the patterns' cumulative steps and multiplied four sites at a time (dp4a).
+constexpr int walk_threads(bool corr) { return corr ? 768 : 1024; }  // 85 and 64 registers
+
+template <bool CORR>
+__global__ void __launch_bounds__(walk_threads(CORR), 1)
+walk_kernel(const uint32_t* __restrict__ sys, const uint32_t* __restrict__ snap, int lx, int ly,
+            const int4* __restrict__ rowinfo, const int64_t* __restrict__ rowstart, Partial* __restrict__ partials,
+            Partial* __restrict__ out, WalkState* ws)
+{
+    constexpr int NT = walk_threads(CORR), NWARP = NT / 32;
+    extern __shared__ __align__(16) uint32_t hist[];  // [height bin][pattern ^ bin]
+    __shared__ uint2 lut[CORR ? WALK_LUT : 1];
+    __shared__ long long base_s[CORR ? 2 : 1][AN_MAX_BLOCKS];
+    __shared__ int used[2];  // first and last bin of a chunk's first group
+    __shared__ bool last;
+
+    const uint64_t Wr = 1ull << (lx - 6);
+    const uint64_t Q = 1ull << (lx + ly - 6);
+    const uint64_t rows = 1ull << ly;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int par = (int)(blockIdx.x & 1);            // row parity of this CTA
+    const uint64_t nctas = gridDim.x >> 1, cta = blockIdx.x >> 1;
+    const int64_t* rowstart_s = rowstart + rows;
+    const int4* rowinfo_s = rowinfo + rows;
+
+    if (threadIdx.x == 0) {
+        used[0] = WALK_BINS;
+        used[1] = -1;
+    }
+    for (int i = threadIdx.x; i < WALK_BINS * 64; i += NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (CORR && threadIdx.x < WALK_LUT) {
+        // byte j: 8 + sum_{k <= j} (2 bit_k - 1), the pattern's even-x bits low, odd-x bits high
+        int cum = 8;
+        uint32_t w[2] = {0u, 0u};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            cum += 2 * (int)((threadIdx.x >> ((j & 1 ? 4 : 0) + (j >> 1))) & 1u) - 1;
+            w[j >> 2] |= (uint32_t)cum << (8 * (j & 3));
+        }
+        lut[threadIdx.x] = make_uint2(w[0], w[1]);
+    }
+    const int lgb = row_block_lg(ly), nblk = (int)(rows >> lgb);
+    const long long mid = row_block_bases<NT>(ws->block[0], nblk, base_s[0]);
+    const long long mid_s = CORR ? row_block_bases<NT>(ws->block[1], nblk, base_s[CORR ? 1 : 0]) : 0;
+    // bin s holds groups with height H0 + 2 s before their first site; H0 has the parity of the
+    // heights before x = 0 of this CTA's rows, Hs(y) - e0
+    const long long first_h = rowstart[par] - 1;  // block 0 starts at 0; e0 = +-1: either way the same parity
+    const long long H0 = mid - WALK_BINS + ((mid - WALK_BINS - first_h) & 1);
+    __syncthreads();
+
+    Sums slow{0, 0, 0x7fffffffffffffffll, -0x7fffffffffffffffll, {0, 0, 0, 0, 0}};
+    int bin_lo = WALK_BINS, bin_hi = -1;
+    // correlator: sums over sites of u v and of v, u = h - mid + 128 and v = h' - mid' + 128
+    long long uv_sum = 0, v_sum = 0, agree = 0;
+
+    const int wl = (int)(Wr < 32 ? Wr : 32);      // lanes per row
+    const int rpw = 32 / wl;                      // rows per warp
+    const int parts = Wr >= AN_PART_WORDS ? 4 : 1;
+    const uint64_t pw = Wr / parts;               // words per part
+    const uint64_t items = rows / 2 / rpw * parts;
+    const int sub = lane % wl;
+    const uint64_t be = par ? 2 * Q : 0, bo = par ? 0 : 2 * Q;
+
+    for (uint64_t it = cta * NWARP + wid; it < items; it += nctas * NWARP) {
+        const int part = (int)(it % parts);
+        const uint64_t y = 2 * (it / parts * rpw + lane / wl) + par;
+        const uint64_t off = y * Wr + part * pw;
+        const uint32_t *pe = sys + be + off, *po = sys + bo + off;
+        const uint32_t *qe = snap + be + off, *qo = snap + bo + off;
+        // the next chunk's words: X of both sublattices, for the correlator Y and the snapshot's
+        uint32_t w[CORR ? 8 : 2];
+        auto load = [&](uint64_t c) {
+            w[0] = pe[c];
+            w[1] = po[c];
+            if (CORR) {
+                w[2] = qe[c];
+                w[3] = qo[c];
+                w[4] = pe[Q + c];
+                w[5] = po[Q + c];
+                w[6] = qe[Q + c];
+                w[7] = qo[Q + c];
+            }
+        };
+        load(sub);
+        // height before the part's first site: Hs - e0 + 2 (bits set before it) - sites
+        auto before = [&](const int4& r) { return part == 0 ? 0 : part == 1 ? r.x : part == 2 ? r.y : r.z; };
+        const long long back = (long long)(64 * pw * part);
+        const int4 ri = rowinfo[y];
+        const long long Hs = rowstart[y] + base_s[0][y >> lgb];
+        long long H = Hs - (2 * (int)(sys[be + y * Wr] & 1u) - 1) + 2 * (long long)before(ri) - back;
+        long long Hsn = 0;
+        int sum_s = 0;
+        if (CORR) {
+            const int4 si = rowinfo_s[y];
+            sum_s = row_sum(si.w);
+            Hsn = rowstart_s[y] + base_s[CORR ? 1 : 0][y >> lgb] - (2 * (int)(snap[be + y * Wr] & 1u) - 1) +
+                  2 * (long long)before(si) - back;
+        }
+        const int sum_r = row_sum(ri.w);
+        for (uint64_t c = sub; c < pw; c += wl) {
+            const uint32_t e = w[0], o = w[1];
+            uint32_t es = 0, os = 0;
+            if (CORR) {
+                es = w[2];
+                os = w[3];
+                agree += 2 * (__popc(~(e ^ es)) + __popc(~(o ^ os)) + __popc(~(w[4] ^ w[6])) + __popc(~(w[5] ^ w[7]))) - 128;
+            }
+            if (c + wl < pw) load(c + wl);
+            // the chunk's total step and the heights before it, in the row's lanes
+            const int n = __popc(e) + __popc(o) - 32;
+            int incl = n;
+            int ns = 0, incl_s = 0;
+            if (CORR) incl_s = ns = __popc(es) + __popc(os) - 32;
+            for (int k = 1; k < wl; k <<= 1) {
+                const int a = __shfl_up_sync(0xffffffffu, incl, k, wl);
+                if (sub >= k) incl += a;
+                if (CORR) {
+                    const int b = __shfl_up_sync(0xffffffffu, incl_s, k, wl);
+                    if (sub >= k) incl_s += b;
+                }
+            }
+            const long long h0 = H + 2 * (incl - n);
+            H += 2 * __shfl_sync(0xffffffffu, incl, wl - 1, wl);
+            // patterns of the even and the odd groups, a byte each, and their set bits
+            const uint32_t A = (e & 0x0F0F0F0Fu) | ((o & 0x0F0F0F0Fu) << 4);
+            const uint32_t B = ((e >> 4) & 0x0F0F0F0Fu) | (o & 0xF0F0F0F0u);
+            const uint32_t pa = byte_popc(A), pb = byte_popc(B);
+            const bool open_row = part == 0 && c == 0 && sum_r != 0;
+            const long long rel = h0 - mid;
+            if (rel >= -WALK_REACH && rel < WALK_REACH && !open_row) {
+                // absolute bin of each group: s0 + bits before it - 4 per group before it
+                const int s0 = (int)(h0 - H0) >> 1;
+                bin_lo = min(bin_lo, s0);
+                bin_hi = max(bin_hi, s0);
+                const uint32_t sa = (pa + pb) * 0x01010100u + (uint32_t)s0 * 0x01010101u - 0x18100800u;
+                const uint32_t sb = sa + pa - 0x04040404u;
+                // the pattern is XORed with the bin so that equal patterns at different heights
+                // lie in different banks
+                const uint32_t xa = A ^ sa, xb = B ^ sb;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t ta = __byte_perm(xa, sa, i ? 0x7362 : 0x5140);
+                    const uint32_t tb = __byte_perm(xb, sb, i ? 0x7362 : 0x5140);
+                    atomicAdd(&hist[ta & 0xFFFFu], 1u);
+                    atomicAdd(&hist[tb & 0xFFFFu], 1u);
+                    atomicAdd(&hist[ta >> 16], 1u);
+                    atomicAdd(&hist[tb >> 16], 1u);
+                }
+            } else {
+                long long h = h0;
+#pragma unroll 1
+                for (int i = 0; i < 64; ++i) {
+                    h += 2 * (long long)((((i & 1) ? o : e) >> (i >> 1)) & 1u) - 1;
+                    slow.add_height(i == 0 && open_row ? Hs + sum_r : h);
+                }
+            }
+            if (CORR) {
+                const long long hs0 = Hsn + 2 * (incl_s - ns);
+                Hsn += 2 * __shfl_sync(0xffffffffu, incl_s, wl - 1, wl);
+                const long long rel_s = hs0 - mid_s;
+                const bool open_s = part == 0 && c == 0 && sum_s != 0;
+                // u and v as bytes: no carry while the chunk stays within [-127, 127] of the middles
+                if (rel >= -63 && rel <= 63 && rel_s >= -63 && rel_s <= 63 && !open_row && !open_s) {
+                    const uint32_t As = (es & 0x0F0F0F0Fu) | ((os & 0x0F0F0F0Fu) << 4);
+                    const uint32_t Bs = ((es >> 4) & 0x0F0F0F0Fu) | (os & 0xF0F0F0F0u);
+                    uint32_t b = (uint32_t)((int)rel + 120) * 0x01010101u, bs = (uint32_t)((int)rel_s + 120) * 0x01010101u;
+                    unsigned int uv = 0, vv = 0;
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) {
+                        const uint2 T = lut[((g & 1 ? B : A) >> (8 * (g >> 1))) & 0xFFu];
+                        const uint2 Ts = lut[((g & 1 ? Bs : As) >> (8 * (g >> 1))) & 0xFFu];
+                        const uint32_t u0 = b + T.x, u1 = b + T.y, v0 = bs + Ts.x, v1 = bs + Ts.y;
+                        uv = __dp4a(u0, v0, uv);
+                        uv = __dp4a(u1, v1, uv);
+                        vv = __dp4a(v0, 0x01010101u, vv);
+                        vv = __dp4a(v1, 0x01010101u, vv);
+                        // the next group starts at this one's last height: byte 3, less the 8 of the bias
+                        b = __byte_perm(u1, 0u, 0x3333) - 0x08080808u;
+                        bs = __byte_perm(v1, 0u, 0x3333) - 0x08080808u;
+                    }
+                    uv_sum += uv;
+                    v_sum += vv;
+                } else {
+                    long long r = rel + 128, s = rel_s + 128;
+#pragma unroll 1
+                    for (int i = 0; i < 64; ++i) {
+                        r += 2 * (long long)((((i & 1) ? o : e) >> (i >> 1)) & 1u) - 1;
+                        s += 2 * (long long)((((i & 1) ? os : es) >> (i >> 1)) & 1u) - 1;
+                        // x = 0 takes the height its row ends with
+                        const long long a = i == 0 && part == 0 && c == 0 ? r + sum_r : r;
+                        const long long b = i == 0 && part == 0 && c == 0 ? s + sum_s : s;
+                        uv_sum += a * b;
+                        v_sum += b;
                     }
                 }
             }
         }
     }
-    if constexpr (MODE != 2) {
-        // block reduction in fixed order
-        __shared__ Partial red[AN_THREADS / 32];
-        for (int o = 16; o > 0; o >>= 1) {
-            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-            s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-            cross += __shfl_xor_sync(0xffffffffu, cross, o);
-            agree += __shfl_xor_sync(0xffffffffu, agree, o);
-            ss1 += __shfl_xor_sync(0xffffffffu, ss1, o);
-            hmin = min(hmin, __shfl_xor_sync(0xffffffffu, hmin, o));
-            hmax = max(hmax, __shfl_xor_sync(0xffffffffu, hmax, o));
-            s3 += __shfl_xor_sync(0xffffffffu, s3, o);
-            s4 += __shfl_xor_sync(0xffffffffu, s4, o);
-            s5 += __shfl_xor_sync(0xffffffffu, s5, o);
-            s6 += __shfl_xor_sync(0xffffffffu, s6, o);
-            s7 += __shfl_xor_sync(0xffffffffu, s7, o);
-        }
-        if (lane == 0) {
-            Partial p;
-            p.s1 = s1; p.s2 = s2; p.hmin = hmin; p.hmax = hmax; p.cross = cross; p.agree = agree;
-            p.snap_s1 = ss1; p.pad = 0;
-            p.s[0] = s3; p.s[1] = s4; p.s[2] = s5; p.s[3] = s6; p.s[4] = s7;
-            red[wid] = p;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            Partial p = red[0];
-            for (int w = 1; w < AN_THREADS / 32; ++w) {
-                const Partial& q = red[w];
-                p.s1 += q.s1; p.s2 += q.s2; p.cross += q.cross; p.agree += q.agree;
-                p.snap_s1 += q.snap_s1;
-                p.hmin = min(p.hmin, q.hmin); p.hmax = max(p.hmax, q.hmax);
-                for (int k = 0; k < 5; ++k) p.s[k] += q.s[k];
-            }
-            partials[blockIdx.x] = p;
-        }
+    bin_lo = __reduce_min_sync(0xffffffffu, bin_lo);
+    bin_hi = __reduce_max_sync(0xffffffffu, bin_hi);
+    if (lane == 0) {
+        atomicMin(&used[0], bin_lo);
+        atomicMax(&used[1], bin_hi);
     }
-}
-
-// Sum of the per-CTA partials in a fixed order (so repeated runs agree bit for bit): thread t
-// adds partials t, t + 256, ... in turn, then a fixed pairwise tree over the 256 threads.
-constexpr int FR_THREADS = 256;
-
-__device__ __forceinline__ void merge_partial(Partial& p, const Partial& q)
-{
-    p.s1 += q.s1; p.s2 += q.s2; p.cross += q.cross; p.agree += q.agree;
-    p.snap_s1 += q.snap_s1;
-    p.hmin = min(p.hmin, q.hmin); p.hmax = max(p.hmax, q.hmax);
-    for (int k = 0; k < 5; ++k) p.s[k] += q.s[k];
-}
-
-__global__ void __launch_bounds__(FR_THREADS) final_reduce_kernel(const Partial* __restrict__ partials, int n,
-                                                                  Partial* out)
-{
-    __shared__ Partial red[FR_THREADS];
-    Partial p{};
-    p.hmin = 0x7fffffffffffffffll;
-    p.hmax = -0x7fffffffffffffffll;
-    for (int i = threadIdx.x; i < n; i += FR_THREADS) merge_partial(p, partials[i]);
-    red[threadIdx.x] = p;
     __syncthreads();
-    for (int w = FR_THREADS / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) merge_partial(red[threadIdx.x], red[threadIdx.x + w]);
-        __syncthreads();
+    Partial acc = empty_partial();
+    // thread: pattern p, every (NT / 256)th height bin of those in use (a chunk's later groups
+    // start at most 28 bins from its first)
+    {
+        const int p = (int)(threadIdx.x & 255u);
+        const int end = min(used[1] + 29, WALK_BINS);
+        unsigned long long n0 = 0, n1 = 0, n2 = 0;  // sums of n, n s, n s^2
+        double m3 = 0, m4 = 0, m5 = 0, m6 = 0, m7 = 0;
+        int smin = WALK_BINS, smax = -1;
+        for (int s = max(used[0] - 28, 0) + (int)(threadIdx.x >> 8); s < end; s += NT / 256) {
+            const uint32_t n = hist[s * 256 + (p ^ s)];
+            if (n == 0u) continue;
+            smin = min(smin, s);
+            smax = s;
+            n0 += n;
+            n1 += (unsigned long long)n * (uint32_t)s;
+            n2 += (unsigned long long)n * (uint32_t)(s * s);
+            const double d = (double)(H0 + 2 * s), d2 = d * d, N = (double)n * (d2 * d);
+            m3 += N;
+            m4 += N * d;
+            m5 += N * d2;
+            m6 += N * (d2 * d);
+            m7 += N * (d2 * d2);
+        }
+        if (smax >= 0) {
+            const long long m0 = (long long)n0, m1 = H0 * m0 + 2 * (long long)n1;
+            const long long m2 = H0 * H0 * m0 + 4 * H0 * (long long)n1 + 4 * (long long)n2;
+            int d = 0, dmin = 8, dmax = -8, t[8] = {8, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                d += 2 * ((p >> ((j & 1 ? 4 : 0) + (j >> 1))) & 1) - 1;
+                dmin = min(dmin, d);
+                dmax = max(dmax, d);
+                int f = 1;
+#pragma unroll
+                for (int k = 1; k < 8; ++k) t[k] += (f *= d);
+            }
+            acc.s1 = 8 * m1 + t[1] * m0;
+            acc.s2 = 8 * m2 + 2 * t[1] * m1 + t[2] * m0;
+            acc.hmin = H0 + 2 * smin + dmin;
+            acc.hmax = H0 + 2 * smax + dmax;
+            const double M[8] = {(double)m0, (double)m1, (double)m2, m3, m4, m5, m6, m7};
+            const double T[8] = {8.0,          (double)t[1], (double)t[2], (double)t[3],
+                                 (double)t[4], (double)t[5], (double)t[6], (double)t[7]};
+#pragma unroll
+            for (int k = 3; k < 8; ++k) {
+                double sum = 0.0;
+                int binom = 1;
+#pragma unroll
+                for (int j = 0; j <= k; ++j) {
+                    sum += (double)binom * T[j] * M[k - j];
+                    binom = binom * (k - j) / (j + 1);
+                }
+                acc.s[k - 3] = sum;
+            }
+        }
     }
-    if (threadIdx.x == 0) *out = red[0];
+    acc.s1 += slow.s1;
+    acc.s2 += slow.s2;
+    acc.hmin = min(acc.hmin, slow.hmin);
+    acc.hmax = max(acc.hmax, slow.hmax);
+    for (int k = 0; k < 5; ++k) acc.s[k] += slow.s[k];
+    if (CORR) {
+        // summed over all sites, sum h h' = sum u v + (mid - 128) sum v + (mid' - 128) sum h; the
+        // last term is linear in s1, so every thread adds its share of it
+        acc.cross = uv_sum + (mid - 128) * v_sum + (mid_s - 128) * acc.s1;
+        acc.agree = agree;
+        acc.snap_s1 = v_sum;  // less (128 - mid') per site, below
+    }
+    __syncthreads();  // the counts have been read: their memory takes the values to add up
+    long long* buf = reinterpret_cast<long long*>(hist);
+    cta_partial<NT>(acc, buf, &partials[blockIdx.x]);
+    if (threadIdx.x == 0) {
+        __threadfence();  // the CTA's partial, ordered before this by the barrier
+        last = atomicAdd(&ws->ticket, 1u) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
+    static_assert(AN_MAX_GRID <= NT, "one partial per thread");
+    acc = empty_partial();
+    if (threadIdx.x < gridDim.x) {
+        const longlong2* q = reinterpret_cast<const longlong2*>(partials + threadIdx.x);
+        longlong2* d = reinterpret_cast<longlong2*>(&acc);
+#pragma unroll
+        for (int k = 0; k < (int)(sizeof(Partial) / 16); ++k) d[k] = __ldcg(q + k);
+    }
+    cta_partial<NT>(acc, buf, out);
+    if (CORR && threadIdx.x == 0) out->snap_s1 += (mid_s - 128) * (long long)(rows << lx);
+}
+
+// {Hs(y) - c, h(0, y) - c} of every row, from the row tables of the lattice measured last.
+__global__ void __launch_bounds__(AN_ROW_THREADS)
+row_heights_kernel(const int4* __restrict__ rowinfo, const int64_t* __restrict__ rowstart, int ly, int64_t c,
+                   const WalkState* __restrict__ ws, int2* __restrict__ out)
+{
+    __shared__ long long base_s[AN_MAX_BLOCKS];
+    const uint64_t rows = 1ull << ly;
+    const int lgb = row_block_lg(ly);
+    row_block_bases<AN_ROW_THREADS>(ws->block[0], (int)(rows >> lgb), base_s);
+    for (uint64_t y = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; y < rows; y += (uint64_t)gridDim.x * blockDim.x) {
+        const int64_t h = rowstart[y] + base_s[y >> lgb] - c;
+        out[y] = make_int2((int32_t)h, (int32_t)(h + row_sum(rowinfo[y].w)));
+    }
 }
 
 cudaError_t analysis_alloc(AnalysisScratch* s, int ly)
@@ -335,11 +644,11 @@ cudaError_t analysis_alloc(AnalysisScratch* s, int ly)
     const size_t rows = 1ull << ly;
     s->rows_cap = rows;
     cudaError_t e;
-    // two row tables (system and snapshot) and partials + final record
-    if ((e = cudaMalloc(&s->rowinfo, 4 * rows * sizeof(int32_t))) != cudaSuccess) return e;
+    // two row tables (system and snapshot) and partials, final record and the walk's state
+    if ((e = cudaMalloc(&s->rowinfo, 2 * rows * sizeof(int4))) != cudaSuccess) return e;
     if ((e = cudaMalloc(&s->rowstart, 2 * rows * sizeof(int64_t))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&s->acc, (AN_MAX_GRID + 1) * sizeof(Partial) + 64)) != cudaSuccess) return e;
-    return cudaSuccess;
+    const size_t acc = (AN_MAX_GRID + 1) * sizeof(Partial) + sizeof(WalkState);
+    return cudaMalloc(&s->acc, acc);
 }
 
 void analysis_free(AnalysisScratch* s)
@@ -350,24 +659,6 @@ void analysis_free(AnalysisScratch* s)
     s->rowinfo = nullptr;
     s->rowstart = nullptr;
     s->acc = nullptr;
-}
-
-static int walk_grid(int lx, int ly)
-{
-    const uint64_t Wr = 1ull << (lx - 6);
-    const int TPR = (int)(Wr < AN_THREADS ? Wr : AN_THREADS);
-    const uint64_t groups = (1ull << ly) / (AN_THREADS / TPR);
-    return (int)(groups < AN_MAX_GRID ? groups : AN_MAX_GRID);
-}
-
-static cudaError_t row_tables(const uint32_t* d, int lx, int ly, int32_t* ri, int64_t* rs,
-                              cudaStream_t st)
-{
-    const uint64_t rows = 1ull << ly;
-    const int grid = (int)((rows * 32 + 255) / 256 < 4096 ? (rows * 32 + 255) / 256 : 4096);
-    rowinfo_kernel<<<grid, 256, 0, st>>>(d, lx, ly, ri);
-    rowstart_kernel<<<1, 1024, 0, st>>>(ri, ly, rs);
-    return cudaGetLastError();
 }
 
 size_t analysis_record_bytes() { return sizeof(Partial); }
@@ -386,77 +677,58 @@ void analysis_decode_record(const void* rec, MomentsOut* out)
     out->snap_s1 = h.snap_s1;
 }
 
+static WalkState* walk_state(AnalysisScratch* s)
+{
+    return reinterpret_cast<WalkState*>(reinterpret_cast<Partial*>(s->acc) + AN_MAX_GRID + 1);
+}
+
+static void launch_rows(const uint32_t* d_sys, const uint32_t* d_snap, int lx, int ly, AnalysisScratch* s,
+                        bool starts, cudaStream_t st)
+{
+    const dim3 grid(1u << (ly - row_block_lg(ly)), d_snap ? 2 : 1);
+    row_kernel<<<grid, AN_ROW_THREADS, 0, st>>>(d_sys, d_snap, lx, ly, s->rowinfo, starts ? s->rowstart : nullptr,
+                                                walk_state(s));
+}
+
 cudaError_t analysis_moments_record(const uint32_t* d_sys, const uint32_t* d_snap, int lx, int ly,
                                     AnalysisScratch* s, void* d_rec, cudaStream_t st)
 {
-    const uint64_t rows = 1ull << ly;
-    int32_t* ri = s->rowinfo;
-    int32_t* ri_s = s->rowinfo + 2 * rows;
-    int64_t* rs = s->rowstart;
-    int64_t* rs_s = s->rowstart + rows;
-    Partial* parts = reinterpret_cast<Partial*>(s->acc);
-    cudaError_t e = row_tables(d_sys, lx, ly, ri, rs, st);
+    launch_rows(d_sys, d_snap, lx, ly, s, true, st);
+    // CTAs per row parity, at most half the SMs
+    const uint64_t Wr = 1ull << (lx - 6);
+    const uint64_t items = Wr >= AN_PART_WORDS ? (1ull << ly) * 2 : (1ull << ly) / 2 / (Wr < 32 ? 32 / Wr : 1);
+    const unsigned threads = walk_threads(d_snap != nullptr);
+    const uint64_t want = (items + threads / 32 - 1) / (threads / 32);
+    const unsigned grid = 2 * (unsigned)(want < AN_MAX_GRID / 2 ? want : AN_MAX_GRID / 2);
+    auto kern = d_snap ? walk_kernel<true> : walk_kernel<false>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_SMEM);
     if (e != cudaSuccess) return e;
-    const int grid = walk_grid(lx, ly);
-    if (d_snap) {
-        if ((e = row_tables(d_snap, lx, ly, ri_s, rs_s, st)) != cudaSuccess) return e;
-        walk_kernel<1><<<grid, AN_THREADS, 0, st>>>(d_sys, d_snap, lx, ly, ri, rs, ri_s, rs_s,
-                                                    nullptr, parts);
-    } else {
-        walk_kernel<0><<<grid, AN_THREADS, 0, st>>>(d_sys, nullptr, lx, ly, ri, rs, nullptr,
-                                                    nullptr, nullptr, parts);
-    }
-    final_reduce_kernel<<<1, FR_THREADS, 0, st>>>(parts, grid, reinterpret_cast<Partial*>(d_rec));
+    kern<<<grid, threads, WALK_SMEM, st>>>(d_sys, d_snap, lx, ly, s->rowinfo, s->rowstart,
+                                           reinterpret_cast<Partial*>(s->acc), reinterpret_cast<Partial*>(d_rec),
+                                           walk_state(s));
+    return cudaGetLastError();
+}
+
+cudaError_t analysis_row_heights(AnalysisScratch* s, int ly, int64_t c, int2* d_out, cudaStream_t st)
+{
+    const uint64_t rows = 1ull << ly;
+    const unsigned grid = (unsigned)(rows / AN_ROW_THREADS < 592 ? rows / AN_ROW_THREADS + 1 : 592);
+    row_heights_kernel<<<grid, AN_ROW_THREADS, 0, st>>>(s->rowinfo, s->rowstart, ly, c, walk_state(s), d_out);
     return cudaGetLastError();
 }
 
 cudaError_t analysis_moments(const uint32_t* d_sys, const uint32_t* d_snap, int lx, int ly,
                              AnalysisScratch* s, MomentsOut* out, cudaStream_t st)
 {
-    const uint64_t rows = 1ull << ly;
-    int32_t* ri = s->rowinfo;
-    int32_t* ri_s = s->rowinfo + 2 * rows;
-    int64_t* rs = s->rowstart;
-    int64_t* rs_s = s->rowstart + rows;
-    Partial* parts = reinterpret_cast<Partial*>(s->acc);
-    Partial* fin = parts + AN_MAX_GRID;
-    cudaError_t e = row_tables(d_sys, lx, ly, ri, rs, st);
+    Partial* fin = reinterpret_cast<Partial*>(s->acc) + AN_MAX_GRID;
+    cudaError_t e = analysis_moments_record(d_sys, d_snap, lx, ly, s, fin, st);
     if (e != cudaSuccess) return e;
-    const int grid = walk_grid(lx, ly);
-    if (d_snap) {
-        if ((e = row_tables(d_snap, lx, ly, ri_s, rs_s, st)) != cudaSuccess) return e;
-        walk_kernel<1><<<grid, AN_THREADS, 0, st>>>(d_sys, d_snap, lx, ly, ri, rs, ri_s, rs_s,
-                                                    nullptr, parts);
-    } else {
-        walk_kernel<0><<<grid, AN_THREADS, 0, st>>>(d_sys, nullptr, lx, ly, ri, rs, nullptr,
-                                                    nullptr, nullptr, parts);
-    }
-    final_reduce_kernel<<<1, FR_THREADS, 0, st>>>(parts, grid, fin);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     Partial h;
     if ((e = cudaMemcpyAsync(&h, fin, sizeof(Partial), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
         return e;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-    out->s1 = h.s1;
-    out->s2 = h.s2;
-    for (int k = 0; k < 5; ++k) out->s3to7[k] = h.s[k];
-    out->hmin = h.hmin;
-    out->hmax = h.hmax;
-    out->cross = h.cross;
-    out->agree = h.agree;
-    out->snap_s1 = h.snap_s1;
+    analysis_decode_record(&h, out);
     return cudaSuccess;
-}
-
-cudaError_t analysis_heights(const uint32_t* d_sys, int lx, int ly, AnalysisScratch* s,
-                             int32_t* d_heights, cudaStream_t st)
-{
-    cudaError_t e = row_tables(d_sys, lx, ly, s->rowinfo, s->rowstart, st);
-    if (e != cudaSuccess) return e;
-    walk_kernel<2><<<walk_grid(lx, ly), AN_THREADS, 0, st>>>(d_sys, nullptr, lx, ly, s->rowinfo,
-                                                             s->rowstart, nullptr, nullptr,
-                                                             d_heights, nullptr);
-    return cudaGetLastError();
 }
 
 // ---- invariants ----
@@ -492,7 +764,7 @@ __global__ void colsum_kernel(const uint32_t* __restrict__ sys, int lx, int ly, 
 }
 
 __global__ void invariants_kernel(const uint32_t* __restrict__ sys, int lx, int ly,
-                                  const int32_t* __restrict__ rowinfo, const int* __restrict__ colsum,
+                                  const int4* __restrict__ rowinfo, const int* __restrict__ colsum,
                                   unsigned long long* rep)
 {
     const uint64_t Wr = 1ull << (lx - 6);
@@ -502,7 +774,7 @@ __global__ void invariants_kernel(const uint32_t* __restrict__ sys, int lx, int 
     unsigned long long badr = 0, badc = 0, badp = 0;
     const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t y = tid; y < rows; y += nth) badr += rowinfo[2 * y + 1] != 0;
+    for (uint64_t y = tid; y < rows; y += nth) badr += row_sum(rowinfo[y].w) != 0;
     for (uint64_t x = tid; x < L; x += nth) badc += colsum[x] != 0;
     // plaquettes: per (sublattice, row, word)
     for (uint64_t i = tid; i < 2 * Q; i += nth) {
@@ -536,14 +808,13 @@ __global__ void invariants_kernel(const uint32_t* __restrict__ sys, int lx, int 
 cudaError_t analysis_invariants(const uint32_t* d_sys, int lx, int ly, AnalysisScratch* s,
                                 int64_t rep[3], cudaStream_t st)
 {
-    const uint64_t rows = 1ull << ly, L = 1ull << lx;
+    const uint64_t L = 1ull << lx;
     int* colsum = nullptr;
     cudaError_t e;
     if ((e = cudaMallocAsync(&colsum, L * sizeof(int) + 64, st)) != cudaSuccess) return e;
     unsigned long long* drep = reinterpret_cast<unsigned long long*>(colsum + L);
     cudaMemsetAsync(colsum, 0, L * sizeof(int) + 64, st);
-    const int grid0 = (int)((rows * 32 + 255) / 256 < 4096 ? (rows * 32 + 255) / 256 : 4096);
-    rowinfo_kernel<<<grid0, 256, 0, st>>>(d_sys, lx, ly, s->rowinfo);
+    launch_rows(d_sys, nullptr, lx, ly, s, false, st);
     colsum_kernel<<<512, 256, 0, st>>>(d_sys, lx, ly, colsum);
     invariants_kernel<<<1184, 256, 0, st>>>(d_sys, lx, ly, s->rowinfo, colsum, drep);
     unsigned long long h[3] = {0, 0, 0};
@@ -585,9 +856,9 @@ cudaError_t analysis_invariants(const uint32_t* d_sys, int lx, int ly, AnalysisS
 namespace kpzb {
 
 constexpr int NOALLOC_MAX_LY = 16;
-constexpr size_t NOALLOC_ROWINFO = 2ull * (1ull << NOALLOC_MAX_LY) * sizeof(int32_t);
+constexpr size_t NOALLOC_ROWINFO = (1ull << NOALLOC_MAX_LY) * sizeof(int4);
 constexpr size_t NOALLOC_ROWSTART = (1ull << NOALLOC_MAX_LY) * sizeof(int64_t);
-constexpr size_t NOALLOC_PARTIALS = (AN_MAX_GRID + 1) * sizeof(Partial);
+constexpr size_t NOALLOC_PARTIALS = (AN_MAX_GRID + 1) * sizeof(Partial) + sizeof(WalkState);
 constexpr size_t NOALLOC_BYTES = NOALLOC_ROWINFO + NOALLOC_ROWSTART + NOALLOC_PARTIALS;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
@@ -673,7 +944,7 @@ extern "C" kpzb_status kpzb_roughness_noalloc(const uint32_t* d_cbbit, int lx, i
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(no-alloc scratch)");
     unsigned char* base = static_cast<unsigned char*>(addr);
     AnalysisScratch view;
-    view.rowinfo = reinterpret_cast<int32_t*>(base);
+    view.rowinfo = reinterpret_cast<int4*>(base);
     view.rowstart = reinterpret_cast<int64_t*>(base + NOALLOC_ROWINFO);
     view.acc = reinterpret_cast<unsigned long long*>(base + NOALLOC_ROWINFO + NOALLOC_ROWSTART);
     view.rows_cap = 1ull << NOALLOC_MAX_LY;

@@ -74,6 +74,10 @@ struct kpzb_handle {
     void* d_rough = nullptr;
     void* h_rough = nullptr;
     bool rough_pending = false;
+    // records of a measurement run: kept, since a pool allocation per run was given back at the
+    // next synchronisation and cost more than the run's kernels at 8192^2
+    unsigned char* d_rec = nullptr;
+    size_t rec_bytes = 0;
     double pc[4] = {1.0, 1.0, 1.0, 1.0}, qc[4] = {0.0, 0.0, 0.0, 0.0};
     bool class_set[4] = {true, false, false, false};
     AnalysisScratch an{};
@@ -175,6 +179,7 @@ extern "C" kpzb_status kpzb_destroy(kpzb_handle* h)
     cudaFree(h->d_counters);
     cudaFree(h->d_dis);
     cudaFree(h->d_rough);
+    cudaFree(h->d_rec);
     if (h->h_rough) cudaFreeHost(h->h_rough);
     if (h->an.rowinfo) analysis_free(&h->an);
     dt_free(&h->dt);
@@ -943,8 +948,14 @@ extern "C" kpzb_status kpzb_measure_run(kpzb_handle* h, const kpzb_sampling* s, 
     if (times.empty()) return KPZB_OK;
 
     const size_t rb = analysis_record_bytes();
-    unsigned char* d_rec = nullptr;
-    KPZB_CU(cudaMallocAsync(&d_rec, rb * times.size(), h->st), "cudaMallocAsync(records)");
+    if (h->rec_bytes < rb * times.size()) {
+        cudaFree(h->d_rec);
+        h->d_rec = nullptr;
+        h->rec_bytes = 0;
+        KPZB_CU(cudaMalloc(&h->d_rec, rb * times.size()), "cudaMalloc(records)");
+        h->rec_bytes = rb * times.size();
+    }
+    unsigned char* const d_rec = h->d_rec;
     if (tag && !h->d_snap) KPZB_CU(cudaMalloc(&h->d_snap, h->words() * 4), "cudaMalloc(snapshot)");
     kpzb_status rs = KPZB_OK;
     int snap_row = -1;
@@ -967,7 +978,6 @@ extern "C" kpzb_status kpzb_measure_run(kpzb_handle* h, const kpzb_sampling* s, 
     }
     std::vector<unsigned char> host(rb * times.size());
     cudaError_t e = cudaMemcpyAsync(host.data(), d_rec, host.size(), cudaMemcpyDeviceToHost, h->st);
-    cudaFreeAsync(d_rec, h->st);
     kpzb_status js = kpzb_join(h);  // also reports a bounded device wait that expired
     if (rs != KPZB_OK) return rs;
     if (e != cudaSuccess) return cuda_fail(e, "measurement records");

@@ -34,15 +34,6 @@
 
 namespace kpzb {
 
-// per-row data of snapshot s: {b(y), z(y)} = {Hs(y) - c, h(0, y) - c} from the height walk's
-// row starts Hs and row sums (the analysis scratch of the snapshot just measured)
-__global__ void gram_rows_kernel(const int64_t* __restrict__ rowstart, const int32_t* __restrict__ rowinfo,
-                                 uint64_t rows, int64_t c, int2* __restrict__ out)
-{
-    for (uint64_t y = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; y < rows; y += (uint64_t)gridDim.x * blockDim.x)
-        out[y] = make_int2((int32_t)(rowstart[y] - c), (int32_t)(rowstart[y] + rowinfo[2 * y + 1] - c));
-}
-
 // Plain int64 CUDA-core Gram of v = h - c over all snapshot pairs, from the same slope
 // snapshots: a CTA takes a contiguous range of 128-site tiles, its 256 threads rebuild the 64
 // snapshots x 128 sites of each tile into shared memory (gram_slope.cuh, a lane quad per
@@ -197,10 +188,8 @@ extern "C" kpzb_status kpzb_gram_add_device(kpzb_gram* g, const uint32_t* d_cbbi
     uint32_t* dst = g->d_snap + (uint64_t)s * 2 * g->Q;
     GCU(cudaMemcpyAsync(dst, d_cbbit, g->Q * 4, cudaMemcpyDeviceToDevice, g->st), "snapshot copy");
     GCU(cudaMemcpyAsync(dst + g->Q, d_cbbit + 2 * g->Q, g->Q * 4, cudaMemcpyDeviceToDevice, g->st), "snapshot copy");
-    const int grid = (int)std::min<uint64_t>(g->rows / 256 + 1, (uint64_t)g->sm_count * 4);
-    gram_rows_kernel<<<grid, 256, 0, g->st>>>(g->an.rowstart, g->an.rowinfo, g->rows, c,
-                                             g->d_rows + (uint64_t)s * g->rows);
-    GCU(cudaGetLastError(), "gram_rows_kernel");
+    // per-row data {b(y), z(y)} = {Hs(y) - c, h(0, y) - c}
+    GCU(analysis_row_heights(&g->an, g->ly, c, g->d_rows + (uint64_t)s * g->rows, g->st), "snapshot rows");
     GCU(cudaStreamSynchronize(g->st), "snapshot sync");
     g->shift.push_back(c);
     g->s1v.push_back(m.s1 - (int64_t)g->N * c);

@@ -101,9 +101,9 @@ cudaError_t cbbit_to_local_dev(const uint32_t* cbbit, uint32_t* local, int lx, i
 
 // analysis on ENC_CBBIT lattices
 struct AnalysisScratch {
-    int32_t* rowinfo;      // 2 * rows: y-slope step at x=0 and x-slope row sum
-    int64_t* rowstart;     // rows: height at the start of each row walk
-    unsigned long long* acc;  // accumulators (see analysis.cu)
+    int4* rowinfo;         // 2 * rows (system, snapshot): slope counts of each row (see analysis.cu)
+    int64_t* rowstart;     // 2 * rows: height at the start of each row walk, within its row block
+    unsigned long long* acc;  // partial sums and the walk's state (see analysis.cu)
     size_t rows_cap;
 };
 cudaError_t analysis_alloc(AnalysisScratch* s, int ly);
@@ -126,8 +126,9 @@ size_t analysis_record_bytes();
 cudaError_t analysis_moments_record(const uint32_t* d_sys, const uint32_t* d_snap, int lx, int ly,
                                     AnalysisScratch* s, void* d_rec, cudaStream_t st);
 void analysis_decode_record(const void* rec, MomentsOut* out);
-cudaError_t analysis_heights(const uint32_t* d_sys, int lx, int ly, AnalysisScratch* s,
-                             int32_t* d_heights, cudaStream_t st);
+// {Hs(y) - c, h(0, y) - c} of every row of the lattice measured last with s (Hs: the height the
+// walk carries into row y) into d_out[2^ly]
+cudaError_t analysis_row_heights(AnalysisScratch* s, int ly, int64_t c, int2* d_out, cudaStream_t st);
 // invariants: rep[0] bad rows, rep[1] bad columns, rep[2] bad plaquettes
 cudaError_t analysis_invariants(const uint32_t* d_sys, int lx, int ly, AnalysisScratch* s,
                                 int64_t rep[3], cudaStream_t st);

@@ -183,7 +183,7 @@ kpzb_status kpzb_roughness_async(kpzb_handle* h);
 kpzb_status kpzb_roughness_join(kpzb_handle* h, double out[8]);
 /* Roughness (as kpzb_roughness) of a caller's device ENC_CBBIT lattice, without allocating:
  * no cudaMalloc/cudaFree or allocating library call; scratch lives in a fixed device array
- * of about 1.2 MB held by every GPU that loads the library's module.  For callers that
+ * of about 1.6 MB held by every GPU that loads the library's module.  For callers that
  * cannot allocate device memory at measurement time (their allocator owns the device, or an
  * allocation would synchronize the device inside a timing loop).  No counterpart in the
  * reference.  Limit: ly <= 16.  Calls overlapping on the GPU race on the shared scratch.
