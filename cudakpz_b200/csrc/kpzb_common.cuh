@@ -73,51 +73,133 @@ __host__ __device__ inline Thresh make_thresh(uint64_t T)
     return r;
 }
 
+// The first two Philox rounds of a decision's planes, split into what depends on the site group
+// and what depends on the plane.  The planes of one group and half-step share counter words 0, 1
+// and 3 and differ in word 2 alone, so round 1 multiplies the group index and the plane
+// separately, and in round 2 the product with counter word 0 depends only on the plane and the
+// one with word 2 only on the group: the state after round 2 is
+//   { g.a ^ p.x, g.b, g.c ^ p.z, p.w }
+// and a plane costs eight rounds instead of ten.  A round's two 32 x 32 -> 64 bit products take 4.25
+// cycles each per warp and scheduler, twice a logic operation, so rounds are what a plane is
+// made of.  With the comparison below: (0.95,0.05) at 8192^2 49 -> 42 us per MCS, binary disorder at
+// 4096 x 2048 20 -> 15.6 us (a warp runs as many planes as its slowest lane, 12.6 of a mean 7.5).
+struct PlanePart {
+    uint32_t x, z, w;
+};
+struct GroupPart {
+    uint32_t a, b, c;
+};
+__host__ __device__ __forceinline__ PlanePart plane_part(uint32_t plane, uint32_t step, Key k)
+{
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * (plane | (TAG_SCA << 8));
+    const uint64_t p0 = (uint64_t)0xD2511F53u * ((uint32_t)(p1 >> 32) ^ step ^ k.k0);
+    return PlanePart{(uint32_t)p1 ^ (k.k0 + 0x9E3779B9u), (uint32_t)(p0 >> 32) ^ (k.k1 + 0xBB67AE85u), (uint32_t)p0};
+}
+__device__ __forceinline__ GroupPart group_part(uint32_t qgroup, uint32_t stream, Key k)
+{
+    const uint64_t p0 = (uint64_t)0xD2511F53u * qgroup;
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * ((uint32_t)(p0 >> 32) ^ stream ^ k.k1);
+    return GroupPart{(uint32_t)(p1 >> 32), (uint32_t)p1, (uint32_t)p0};
+}
+__device__ __forceinline__ uint4 philox_plane(const GroupPart& g, const PlanePart& p, Key k)
+{
+    uint4 c = make_uint4(g.a ^ p.x, g.b, g.c ^ p.z, p.w);
+    uint32_t k0 = k.k0 + 0x9E3779B9u, k1 = k.k1 + 0xBB67AE85u;
+#pragma unroll
+    for (int r = 2; r < 10; ++r) {
+        k0 += 0x9E3779B9u;
+        k1 += 0xBB67AE85u;
+        const uint64_t p0 = (uint64_t)0xD2511F53u * c.x, p1 = (uint64_t)0xCD9E8D57u * c.z;
+        c = make_uint4((uint32_t)(p1 >> 32) ^ c.y ^ k0, (uint32_t)p1, (uint32_t)(p0 >> 32) ^ c.w ^ k1, (uint32_t)p0);
+    }
+    return c;
+}
+
+// Plane parts of one half-step: all 32 as a table (a kernel parameter), or made as they are needed.
+struct PlaneTable {
+    PlanePart p[32];
+    __device__ __forceinline__ PlanePart at(int k) const { return p[k]; }
+};
+inline PlaneTable make_plane_table(uint32_t step, Key key)
+{
+    PlaneTable t;
+    for (uint32_t k = 0; k < 32; ++k) t.p[k] = plane_part(k, step, key);
+    return t;
+}
+struct PlaneMaker {
+    uint32_t step;
+    Key key;
+    __device__ __forceinline__ PlanePart at(int k) const { return plane_part((uint32_t)k, step, key); }
+};
+
+// Bit-serial comparison of a group's 128 uniforms with their sites' thresholds: `eq` marks the
+// sites whose u still equals the threshold's leading planes, `flip` the outcome of the others.  At
+// each plane an undecided site takes its threshold's bit as its outcome; it is decided there when
+// its own bit differs (1 against 0: u < T), and its outcome then stands.  Three logic operations a
+// word and plane (with separate masks for the two kinds of candidate and their decided flips it was
+// six, and selecting each kind's bits two more).  Planes are fetched while a site is undecided,
+// the first four -- a group has about 64 candidates -- without asking.  TB: threshold bit words
+// of plane k; DROP: sites whose threshold has no 1 bit left below plane k (u < T is then false).
+template <class Planes, class TB, class DROP>
+__device__ __forceinline__ uint4 decide_planes(uint4 eq, uint4 flip, int kmax, Key key, const GroupPart& g,
+                                               const Planes& planes, const TB& tb, const DROP& drop)
+{
+    auto plane = [&](int k) {
+        const uint4 r = philox_plane(g, planes.at(k), key);
+        const uint4 b = tb(k);
+        flip.x = (eq.x & b.x) | (~eq.x & flip.x);
+        flip.y = (eq.y & b.y) | (~eq.y & flip.y);
+        flip.z = (eq.z & b.z) | (~eq.z & flip.z);
+        flip.w = (eq.w & b.w) | (~eq.w & flip.w);
+        eq.x &= ~(b.x ^ r.x);
+        eq.y &= ~(b.y ^ r.y);
+        eq.z &= ~(b.z ^ r.z);
+        eq.w &= ~(b.w ^ r.w);
+        drop(k, eq, flip);
+    };
+    int k = 0;
+    if (kmax >= 4) {
+#pragma unroll
+        for (; k < 4; ++k) plane(k);
+    }
+    for (; k < kmax && (eq.x | eq.y | eq.z | eq.w); ++k) plane(k);
+    // u equal to T in every plane: not below it
+    return make_uint4(flip.x & ~eq.x, flip.y & ~eq.y, flip.z & ~eq.z, flip.w & ~eq.w);
+}
+
 // Four-word decision for the 128 sites of one Philox group (qgroup = qword >> 2).
 // cp: local-minimum candidates, cq: local-maximum candidates. Returns the flip mask.
-__device__ __forceinline__ uint4 decide4(uint4 cp, uint4 cq, Thresh tp, Thresh tq, Key key,
-                                         uint32_t qgroup, uint32_t step, uint32_t stream)
+template <class Planes>
+__device__ __forceinline__ uint4 decide4(uint4 cp, uint4 cq, Thresh tp, Thresh tq, Key key, uint32_t qgroup,
+                                         const Planes& planes, uint32_t stream)
 {
-    uint4 ltp, eqp, ltq, eqq;
-    if (tp.always) {
-        ltp = cp;
-        eqp = make_uint4(0, 0, 0, 0);
-    } else {
-        ltp = make_uint4(0, 0, 0, 0);
-        eqp = tp.planes ? cp : make_uint4(0, 0, 0, 0);
-    }
-    if (tq.always) {
-        ltq = cq;
-        eqq = make_uint4(0, 0, 0, 0);
-    } else {
-        ltq = make_uint4(0, 0, 0, 0);
-        eqq = tq.planes ? cq : make_uint4(0, 0, 0, 0);
-    }
-    const int kmax = max(tp.planes, tq.planes);
-    for (int k = 0; k < kmax; ++k) {
-        const uint32_t any = eqp.x | eqp.y | eqp.z | eqp.w | eqq.x | eqq.y | eqq.z | eqq.w;
-        if (!any) break;
-        const uint4 r = philox4x32_10(make_uint4(qgroup, step, (uint32_t)k | (TAG_SCA << 8), stream), key);
-        const uint32_t bp = (tp.t >> (31 - k)) & 1u;
-        const uint32_t bq = (tq.t >> (31 - k)) & 1u;
-        // bit of T is 1: sites with u-bit 0 are below T (decided), u-bit 1 stay equal.
-        // bit of T is 0: sites with u-bit 1 are above T (drop), u-bit 0 stay equal.
-        if (bp) {
-            ltp.x |= eqp.x & ~r.x; ltp.y |= eqp.y & ~r.y; ltp.z |= eqp.z & ~r.z; ltp.w |= eqp.w & ~r.w;
-            eqp.x &= r.x; eqp.y &= r.y; eqp.z &= r.z; eqp.w &= r.w;
-        } else {
-            eqp.x &= ~r.x; eqp.y &= ~r.y; eqp.z &= ~r.z; eqp.w &= ~r.w;
-        }
-        if (bq) {
-            ltq.x |= eqq.x & ~r.x; ltq.y |= eqq.y & ~r.y; ltq.z |= eqq.z & ~r.z; ltq.w |= eqq.w & ~r.w;
-            eqq.x &= r.x; eqq.y &= r.y; eqq.z &= r.z; eqq.w &= r.w;
-        } else {
-            eqq.x &= ~r.x; eqq.y &= ~r.y; eqq.z &= ~r.z; eqq.w &= ~r.w;
-        }
-        if (k + 1 >= tp.planes) eqp = make_uint4(0, 0, 0, 0);
-        if (k + 1 >= tq.planes) eqq = make_uint4(0, 0, 0, 0);
-    }
-    return make_uint4(ltp.x | ltq.x, ltp.y | ltq.y, ltp.z | ltq.z, ltp.w | ltq.w);
+    const uint32_t ap = tp.always ? 0xFFFFFFFFu : 0u, aq = tq.always ? 0xFFFFFFFFu : 0u;
+    const uint32_t hp = tp.planes ? 0xFFFFFFFFu : 0u, hq = tq.planes ? 0xFFFFFFFFu : 0u;
+    const uint4 eq = make_uint4((cp.x & hp) | (cq.x & hq), (cp.y & hp) | (cq.y & hq), (cp.z & hp) | (cq.z & hq),
+                                (cp.w & hp) | (cq.w & hq));
+    const uint4 flip = make_uint4((cp.x & ap) | (cq.x & aq), (cp.y & ap) | (cq.y & aq), (cp.z & ap) | (cq.z & aq),
+                                  (cp.w & ap) | (cq.w & aq));
+    auto tb = [&](int k) {
+        const uint32_t bp = (uint32_t)((int32_t)(tp.t << k) >> 31), bq = (uint32_t)((int32_t)(tq.t << k) >> 31);
+        return make_uint4((cq.x & bq) | (~cq.x & bp), (cq.y & bq) | (~cq.y & bp), (cq.z & bq) | (~cq.z & bp),
+                          (cq.w & bq) | (~cq.w & bp));
+    };
+    auto drop = [&](int k, uint4& e, uint4& f) {
+        auto out = [&](uint32_t keep_p, uint32_t keep_q) {
+            auto one = [&](uint32_t c, uint32_t& ew, uint32_t& fw) {
+                const uint32_t keep = (c & keep_q) | (~c & keep_p);
+                fw &= ~(ew & ~keep);
+                ew &= keep;
+            };
+            one(cq.x, e.x, f.x);
+            one(cq.y, e.y, f.y);
+            one(cq.z, e.z, f.z);
+            one(cq.w, e.w, f.w);
+        };
+        if (k + 1 == tp.planes) out(0u, 0xFFFFFFFFu);
+        if (k + 1 == tq.planes) out(0xFFFFFFFFu, 0u);
+    };
+    return decide_planes(eq, flip, max(tp.planes, tq.planes), key, group_part(qgroup, stream, key), planes, tb, drop);
 }
 
 // Decision modes, chosen once per launch from the two thresholds:
@@ -154,7 +236,7 @@ __device__ __forceinline__ uint4 decide4_mode(int mode, uint4 cp, uint4 cq, Thre
                           (cp.z & (ap | (hp & ~r.z))) | (cq.z & (aq | (hq & ~r.z))),
                           (cp.w & (ap | (hp & ~r.w))) | (cq.w & (aq | (hq & ~r.w))));
     }
-    return decide4(cp, cq, tp, tq, key, qgroup, step, stream);
+    return decide4(cp, cq, tp, tq, key, qgroup, PlaneMaker{step, key}, stream);
 }
 
 // Quenched disorder (mcsDisorder2SyncRng): every site carries a 2-bit rate class c (bit 0 in
@@ -162,18 +244,20 @@ __device__ __forceinline__ uint4 decide4_mode(int mode, uint4 cp, uint4 cq, Thre
 // same random planes as decide4, so equal rates in every class give decide4's result.
 struct DisorderRates {
     Thresh tp[4], tq[4];
-    int planes;  // most planes any of the eight thresholds can need
+    int planes;            // most planes any of the eight thresholds can need
+    uint32_t last_planes;  // bit k: plane k is the last that one of them can need
 };
 
 inline DisorderRates make_disorder_rates(const uint64_t Tp[4], const uint64_t Tq[4])
 {
     DisorderRates dr{};
-    dr.planes = 0;
     for (int c = 0; c < 4; ++c) {
         dr.tp[c] = make_thresh(Tp[c]);
         dr.tq[c] = make_thresh(Tq[c]);
         if (dr.tp[c].planes > dr.planes) dr.planes = dr.tp[c].planes;
         if (dr.tq[c].planes > dr.planes) dr.planes = dr.tq[c].planes;
+        if (dr.tp[c].planes) dr.last_planes |= 1u << (dr.tp[c].planes - 1);
+        if (dr.tq[c].planes) dr.last_planes |= 1u << (dr.tq[c].planes - 1);
     }
     return dr;
 }
@@ -191,8 +275,9 @@ __device__ __forceinline__ uint32_t dis_word(uint32_t cp, uint32_t cq, uint32_t 
            (cq & sel_class(d0, d1, bq[0], bq[1], bq[2], bq[3]));
 }
 
+template <class Planes>
 __device__ __forceinline__ uint4 decide4_dis(uint4 cp, uint4 cq, uint4 d0, uint4 d1, const DisorderRates& dr,
-                                             Key key, uint32_t qgroup, uint32_t step, uint32_t stream)
+                                             Key key, uint32_t qgroup, const Planes& planes, uint32_t stream)
 {
     uint32_t ap[4], aq[4], hp[4], hq[4];
     for (int c = 0; c < 4; ++c) {
@@ -202,32 +287,44 @@ __device__ __forceinline__ uint4 decide4_dis(uint4 cp, uint4 cq, uint4 d0, uint4
         hq[c] = dr.tq[c].planes ? 0xFFFFFFFFu : 0u;
     }
     // decided flips (threshold 2^32) and sites still equal to their threshold's prefix
-    uint4 lt = make_uint4(dis_word(cp.x, cq.x, d0.x, d1.x, ap, aq), dis_word(cp.y, cq.y, d0.y, d1.y, ap, aq),
-                          dis_word(cp.z, cq.z, d0.z, d1.z, ap, aq), dis_word(cp.w, cq.w, d0.w, d1.w, ap, aq));
-    uint4 eq = make_uint4(dis_word(cp.x, cq.x, d0.x, d1.x, hp, hq), dis_word(cp.y, cq.y, d0.y, d1.y, hp, hq),
-                          dis_word(cp.z, cq.z, d0.z, d1.z, hp, hq), dis_word(cp.w, cq.w, d0.w, d1.w, hp, hq));
-    for (int k = 0; k < dr.planes; ++k) {
-        if (!(eq.x | eq.y | eq.z | eq.w)) break;
-        const uint4 r = philox4x32_10(make_uint4(qgroup, step, (uint32_t)k | (TAG_SCA << 8), stream), key);
-        uint32_t bp[4], bq[4], ep[4], eqn[4];
+    const uint4 flip = make_uint4(dis_word(cp.x, cq.x, d0.x, d1.x, ap, aq), dis_word(cp.y, cq.y, d0.y, d1.y, ap, aq),
+                                  dis_word(cp.z, cq.z, d0.z, d1.z, ap, aq), dis_word(cp.w, cq.w, d0.w, d1.w, ap, aq));
+    const uint4 eq = make_uint4(dis_word(cp.x, cq.x, d0.x, d1.x, hp, hq), dis_word(cp.y, cq.y, d0.y, d1.y, hp, hq),
+                                dis_word(cp.z, cq.z, d0.z, d1.z, hp, hq), dis_word(cp.w, cq.w, d0.w, d1.w, hp, hq));
+    // threshold bit of every site's class and kind of candidate
+    auto pick = [&](const uint32_t bp[4], const uint32_t bq[4]) {
+        auto one = [&](uint32_t c, uint32_t e0, uint32_t e1) {
+            return (c & sel_class(e0, e1, bq[0], bq[1], bq[2], bq[3])) |
+                   (~c & sel_class(e0, e1, bp[0], bp[1], bp[2], bp[3]));
+        };
+        return make_uint4(one(cq.x, d0.x, d1.x), one(cq.y, d0.y, d1.y), one(cq.z, d0.z, d1.z), one(cq.w, d0.w, d1.w));
+    };
+    auto tb = [&](int k) {
+        uint32_t bp[4], bq[4];
         for (int c = 0; c < 4; ++c) {
-            bp[c] = ((dr.tp[c].t >> (31 - k)) & 1u) ? 0xFFFFFFFFu : 0u;
-            bq[c] = ((dr.tq[c].t >> (31 - k)) & 1u) ? 0xFFFFFFFFu : 0u;
-            // thresholds with no 1 bit left below this plane can no longer be exceeded from below
-            ep[c] = (k + 1 >= dr.tp[c].planes) ? 0xFFFFFFFFu : 0u;
-            eqn[c] = (k + 1 >= dr.tq[c].planes) ? 0xFFFFFFFFu : 0u;
+            bp[c] = (uint32_t)((int32_t)(dr.tp[c].t << k) >> 31);
+            bq[c] = (uint32_t)((int32_t)(dr.tq[c].t << k) >> 31);
         }
-#define KPZB_DIS_PLANE(F)                                                   \
-    {                                                                       \
-        const uint32_t tb = dis_word(cp.F, cq.F, d0.F, d1.F, bp, bq);       \
-        lt.F |= eq.F & tb & ~r.F;                                           \
-        eq.F &= ~(tb ^ r.F);                                                \
-        eq.F &= ~dis_word(cp.F, cq.F, d0.F, d1.F, ep, eqn);                 \
-    }
-        KPZB_DIS_PLANE(x) KPZB_DIS_PLANE(y) KPZB_DIS_PLANE(z) KPZB_DIS_PLANE(w)
-#undef KPZB_DIS_PLANE
-    }
-    return lt;
+        return pick(bp, bq);
+    };
+    auto drop = [&](int k, uint4& e, uint4& f) {
+        if (!((dr.last_planes >> k) & 1u)) return;
+        uint32_t kp[4], kq[4];
+        for (int c = 0; c < 4; ++c) {
+            kp[c] = k + 1 == dr.tp[c].planes ? 0u : 0xFFFFFFFFu;
+            kq[c] = k + 1 == dr.tq[c].planes ? 0u : 0xFFFFFFFFu;
+        }
+        const uint4 keep = pick(kp, kq);
+        f.x &= ~(e.x & ~keep.x);
+        f.y &= ~(e.y & ~keep.y);
+        f.z &= ~(e.z & ~keep.z);
+        f.w &= ~(e.w & ~keep.w);
+        e.x &= keep.x;
+        e.y &= keep.y;
+        e.z &= keep.z;
+        e.w &= keep.w;
+    };
+    return decide_planes(eq, flip, dr.planes, key, group_part(qgroup, stream, key), planes, tb, drop);
 }
 
 __device__ __forceinline__ uint4 operator^(uint4 a, uint4 b)

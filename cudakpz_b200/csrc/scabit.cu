@@ -15,6 +15,8 @@
 // with 128-bit loads/stores (one Philox group of 4 words per thread).  Rows longer than
 // one segment are walked segment by segment with the one-bit mask carry kept in shared
 // memory; the carry out of the last word wraps into bit 0 of word 0 (periodic x).
+#include <type_traits>
+
 #include "kpzb_api_internal.h"
 #include "kpzb_common.cuh"
 #include "kpzb_internal.h"
@@ -28,12 +30,14 @@ constexpr int SCABIT_THREADS = 256;
 // bit 0 in the X quadrants, bit 1 in the Y quadrants, i.e. the ENC_LOCAL class words put
 // through the lattice codec), dr the four classes' thresholds (Disorder2SyncRng,
 // kpz/kpzSCACores.cu:217-280).
-template <bool COUNT, bool DIS>
+// GENERAL: rates of more than one random plane (and disorder); their plane parts come as a table.
+struct NoPlanes {};
+template <bool COUNT, bool DIS, bool GENERAL>
 __global__ void __launch_bounds__(SCABIT_THREADS)
 scabit_half_kernel(uint32_t* __restrict__ sys, int lx, int ly, int sigma, uint32_t step, Key key,
                    uint32_t stream, Thresh tp, Thresh tq, int TX, int TY,
                    unsigned long long* __restrict__ counters, const uint32_t* __restrict__ dis,
-                   DisorderRates dr)
+                   DisorderRates dr, const std::conditional_t<GENERAL, PlaneTable, NoPlanes> planes)
 {
     __shared__ uint32_t nxt_s[SCABIT_THREADS];
     __shared__ uint32_t carry_s[2][SCABIT_THREADS];
@@ -89,10 +93,12 @@ scabit_half_kernel(uint32_t* __restrict__ sys, int lx, int ly, int sigma, uint32
             cq.z = tX.z & tY.z & ~(xX.z | oY.z);
             cq.w = tX.w & tY.w & ~(xX.w | oY.w);
             uint4 m;
-            if (DIS) {
+            if constexpr (DIS) {
                 const uint4 d0 = *reinterpret_cast<const uint4*>(dis + bthisX + roff + wi);
                 const uint4 d1 = *reinterpret_cast<const uint4*>(dis + bthisY + roff + wi);
-                m = decide4_dis(cp, cq, d0, d1, dr, key, (uint32_t)((roff + wi) >> 2), step, stream);
+                m = decide4_dis(cp, cq, d0, d1, dr, key, (uint32_t)((roff + wi) >> 2), planes, stream);
+            } else if constexpr (GENERAL) {
+                m = decide4(cp, cq, tp, tq, key, (uint32_t)((roff + wi) >> 2), planes, stream);
             } else {
                 m = decide4_mode(dec_mode(tp, tq), cp, cq, tp, tq, key, (uint32_t)((roff + wi) >> 2), step,
                                  stream);
@@ -165,13 +171,18 @@ cudaError_t scabit_half(uint32_t* d_sys, int lx, int ly, int sigma, uint32_t ste
     const Thresh tp = make_thresh(Tp), tq = make_thresh(Tq);
     dim3 block(sh.TX, sh.TY);
     const DisorderRates dr{};
-    if (d_counters)
-        scabit_half_kernel<true, false><<<sh.grid, block, 0, st>>>(d_sys, lx, ly, sigma, step, key, stream_id,
-                                                                   tp, tq, sh.TX, sh.TY, d_counters, nullptr, dr);
-    else
-        scabit_half_kernel<false, false><<<sh.grid, block, 0, st>>>(d_sys, lx, ly, sigma, step, key, stream_id,
-                                                                    tp, tq, sh.TX, sh.TY, nullptr, nullptr, dr);
-    return cudaGetLastError();
+    auto go = [&](auto kern, const auto& planes) {
+        kern<<<sh.grid, block, 0, st>>>(d_sys, lx, ly, sigma, step, key, stream_id, tp, tq, sh.TX, sh.TY, d_counters,
+                                        nullptr, dr, planes);
+        return cudaGetLastError();
+    };
+    if (dec_mode(tp, tq) == DEC_GENERAL) {
+        const PlaneTable planes = make_plane_table(step, key);
+        return d_counters ? go(scabit_half_kernel<true, false, true>, planes)
+                          : go(scabit_half_kernel<false, false, true>, planes);
+    }
+    return d_counters ? go(scabit_half_kernel<true, false, false>, NoPlanes{})
+                      : go(scabit_half_kernel<false, false, false>, NoPlanes{});
 }
 
 cudaError_t scabit_half_dis(uint32_t* d_sys, const uint32_t* d_dis_cbbit, int lx, int ly, int sigma,
@@ -181,15 +192,11 @@ cudaError_t scabit_half_dis(uint32_t* d_sys, const uint32_t* d_dis_cbbit, int lx
 {
     const Key key = make_key(seed);
     const DisorderRates dr = make_disorder_rates(Tp, Tq);
+    const PlaneTable planes = make_plane_table(step, key);
     dim3 block(sh.TX, sh.TY);
-    if (d_counters)
-        scabit_half_kernel<true, true><<<sh.grid, block, 0, st>>>(d_sys, lx, ly, sigma, step, key, stream_id,
-                                                                  dr.tp[0], dr.tq[0], sh.TX, sh.TY, d_counters,
-                                                                  d_dis_cbbit, dr);
-    else
-        scabit_half_kernel<false, true><<<sh.grid, block, 0, st>>>(d_sys, lx, ly, sigma, step, key, stream_id,
-                                                                   dr.tp[0], dr.tq[0], sh.TX, sh.TY, nullptr,
-                                                                   d_dis_cbbit, dr);
+    auto kern = d_counters ? scabit_half_kernel<true, true, true> : scabit_half_kernel<false, true, true>;
+    kern<<<sh.grid, block, 0, st>>>(d_sys, lx, ly, sigma, step, key, stream_id, dr.tp[0], dr.tq[0], sh.TX, sh.TY,
+                                    d_counters, d_dis_cbbit, dr, planes);
     return cudaGetLastError();
 }
 
