@@ -383,6 +383,19 @@ extern "C" kpzb_status kpzb_autotune(kpzb_handle* h, int* mcs_per_pass, int* cta
     return KPZB_OK;
 }
 
+// Whether the left-over MCS of a call may go through the second buffer: not while the caller
+// captures the stream (nothing may be allocated, and a graph of less than one pass keeps
+// updating the lattice in place), nor when there is no memory for it.
+static bool spare_buffer(kpzb_handle* h)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+    if (ensure_tmp(h) == KPZB_OK) return true;
+    cudaGetLastError();
+    g_err.clear();
+    return false;
+}
+
 static kpzb_status enqueue_sca(kpzb_handle* h, int n)
 {
     const uint64_t Tp = thresh_of(h->p), Tq = thresh_of(h->q);
@@ -445,6 +458,36 @@ static kpzb_status enqueue_sca(kpzb_handle* h, int n)
                 std::swap(h->d_sys, h->d_tmp);
                 done += k;
             }
+        }
+    }
+    // What is left over from whole passes (n mod k): shallower passes of the warp-tile kernel, in
+    // tiles of about the same height, or of the band kernel, which takes any depth.  One pass of r
+    // MCS reads and writes the lattice once where 2r half-step launches do so 2r times: 50 MCS of
+    // 16384^2 at (1,0) end in 27 us instead of 71, 10 MCS of 256^2 in two launches instead of seven.
+    // A lone last MCS of the warp-tile kernel's lattices stays two half-steps.
+    const bool spare = k > 1 && done < n && spare_buffer(h);
+    if (spare && plan.kind == PASS_STRIP) {
+        for (int r = 6; r >= 2; r -= 2) {
+            const int cycle = strip_cycle_rows(r);
+            const int band = (plan.band + 4 * r + cycle / 2) / cycle * cycle - 4 * r;
+            const StripShape rest = scabit_strip_shape(h->lx, h->ly, r, band, mode);
+            if (!rest.ok || r >= k) continue;
+            while (n - done >= r) {
+                KPZB_CU(scabit_strip(h->d_sys, h->d_tmp, h->lx, h->ly, (uint32_t)(h->tdev + done), h->seed,
+                                     h->stream_id, Tp, Tq, rest, cnt, h->st),
+                        "scabit_strip");
+                std::swap(h->d_sys, h->d_tmp);
+                done += r;
+            }
+        }
+    } else if (spare && plan.kind == PASS_BAND && n - done < k) {
+        const FusedShape rest = scabit_fused_shape_cps(h->lx, h->ly, n - done, plan.cps, 0);
+        if (rest.ok) {
+            KPZB_CU(scabit_fused(h->d_sys, h->d_tmp, h->lx, h->ly, (uint32_t)(h->tdev + done), h->seed, h->stream_id,
+                                 Tp, Tq, rest, cnt, reinterpret_cast<unsigned int*>(h->d_counters + 2), h->st),
+                    "scabit_fused");
+            std::swap(h->d_sys, h->d_tmp);
+            done = n;
         }
     }
     for (; done < n; ++done) {

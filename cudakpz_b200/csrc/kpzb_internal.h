@@ -76,7 +76,7 @@ cudaError_t scabit_wave(const uint32_t* d_src, uint32_t* d_dst, int lx, int ly, 
 // warp per tile of a 32-column strip of a quadrant row and a band of rows, the half-steps in
 // registers; strips overlap by two columns (one recomputed column each side).
 struct StripShape {
-    int mcs;           // MCS per pass (4, 6 or 8)
+    int mcs;           // MCS per pass (2, 4, 6 or 8)
     int band;          // output rows per tile
     int nstrips;       // strips per quadrant row
     int ntiles;        // strips x bands (warps)

@@ -255,7 +255,7 @@ StripShape scabit_strip_shape(int lx, int ly, int mcs_per_pass, int band_rows, i
     StripShape s{};
     s.ok = false;
     const int k = mcs_per_pass;
-    if (lx < 11 || lx > 30 || (k != 4 && k != 6 && k != 8)) return s;
+    if (lx < 11 || lx > 30 || (k != 2 && k != 4 && k != 6 && k != 8)) return s;
     if (mode != DEC_NONE && mode != DEC_ONE) return s;
     if (band_rows < 2 || (band_rows & 1)) return s;
     const int64_t Wr = 1ll << (lx - 6);
@@ -294,6 +294,7 @@ static cudaError_t launch_strip(const uint32_t* d_src, uint32_t* d_dst, int lx, 
                                 cudaStream_t st)
 {
     switch (sh.mcs) {
+    case 2: return launch_strip_k<PM, QM, COUNT, 2>(d_src, d_dst, lx, ly, t0, key, stream_id, sh, d_counters, st);
     case 4: return launch_strip_k<PM, QM, COUNT, 4>(d_src, d_dst, lx, ly, t0, key, stream_id, sh, d_counters, st);
     case 6: return launch_strip_k<PM, QM, COUNT, 6>(d_src, d_dst, lx, ly, t0, key, stream_id, sh, d_counters, st);
     case 8: return launch_strip_k<PM, QM, COUNT, 8>(d_src, d_dst, lx, ly, t0, key, stream_id, sh, d_counters, st);
