@@ -34,6 +34,18 @@
 
 namespace kpzb {
 
+// The two X-slope quadrants of a lattice (sublattice 0 at word 0, sublattice 1 at 2Q) into the
+// store's tiles: 16 bytes per tile, smax * 16 apart.
+__global__ void gram_store_kernel(const uint32_t* __restrict__ cbbit, uint64_t Q, int smax, int s, uint4* __restrict__ out)
+{
+    const uint2* a = reinterpret_cast<const uint2*>(cbbit);
+    const uint2* b = reinterpret_cast<const uint2*>(cbbit + 2 * Q);
+    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < Q / 2; t += (uint64_t)gridDim.x * blockDim.x) {
+        const uint2 x = a[t], y = b[t];
+        out[t * (uint64_t)smax + (uint64_t)s] = make_uint4(x.x, x.y, y.x, y.y);
+    }
+}
+
 // Plain int64 CUDA-core Gram of v = h - c over all snapshot pairs, from the same slope
 // snapshots: a CTA takes a contiguous range of 128-site tiles, its 256 threads rebuild the 64
 // snapshots x 128 sites of each tile into shared memory (gram_slope.cuh, a lane quad per
@@ -90,16 +102,17 @@ struct kpzb_gram {
     int lx = 0, ly = 0, device = 0, smax = 0, n = 0, sm_count = 148;
     uint64_t N = 0, Q = 0, rows = 0;
     cudaStream_t st = nullptr;
-    uint32_t* d_snap = nullptr;     // [smax][2][Q] X-slope quadrants
+    uint32_t* d_snap = nullptr;     // X-slope words of every tile and snapshot (gram_slope.cuh)
     int2* d_rows = nullptr;         // [smax][rows] {b(y), z(y)}
     uint32_t* d_tmp = nullptr;      // scratch lattice for host snapshots
     unsigned long long* d_g = nullptr;  // 64 x 64 int64 (CUDA-core path)
     std::vector<int64_t> shift;     // c_s
     std::vector<int64_t> s1v;       // sum (h_s - c_s)
+    int64_t vmin = 0, vmax = 0;     // range of h_s - c_s over the snapshots
     AnalysisScratch an{};
     GramTC tc{};
 
-    SlopeSnapGeom geom() const { return SlopeSnapGeom{d_snap, d_rows, Q, rows, lx, n}; }
+    SlopeSnapGeom geom() const { return SlopeSnapGeom{d_snap, d_rows, Q, rows, lx, smax, n}; }
 };
 
 #define GCHECK(g)                                                       \
@@ -184,13 +197,14 @@ extern "C" kpzb_status kpzb_gram_add_device(kpzb_gram* g, const uint32_t* d_cbbi
     const long double mean = (long double)m.s1 / (long double)g->N;
     const int64_t c = (int64_t)std::floor((double)mean);
     if (m.hmin - c < -1056832 || m.hmax - c > 1040447) return fail(KPZB_EINVAL, "heights exceed three int8 limbs");
-    // the two X-slope quadrants (sublattice 0 at word 0, sublattice 1 at 2Q)
-    uint32_t* dst = g->d_snap + (uint64_t)s * 2 * g->Q;
-    GCU(cudaMemcpyAsync(dst, d_cbbit, g->Q * 4, cudaMemcpyDeviceToDevice, g->st), "snapshot copy");
-    GCU(cudaMemcpyAsync(dst + g->Q, d_cbbit + 2 * g->Q, g->Q * 4, cudaMemcpyDeviceToDevice, g->st), "snapshot copy");
+    const int grid = (int)std::min<uint64_t>(g->Q / 512 + 1, (uint64_t)g->sm_count * 8);
+    gram_store_kernel<<<grid, 256, 0, g->st>>>(d_cbbit, g->Q, g->smax, s, reinterpret_cast<uint4*>(g->d_snap));
+    GCU(cudaGetLastError(), "gram_store_kernel");
     // per-row data {b(y), z(y)} = {Hs(y) - c, h(0, y) - c}
     GCU(analysis_row_heights(&g->an, g->ly, c, g->d_rows + (uint64_t)s * g->rows, g->st), "snapshot rows");
     GCU(cudaStreamSynchronize(g->st), "snapshot sync");
+    g->vmin = std::min<int64_t>(g->vmin, m.hmin - c);
+    g->vmax = std::max<int64_t>(g->vmax, m.hmax - c);
     g->shift.push_back(c);
     g->s1v.push_back(m.s1 - (int64_t)g->N * c);
     g->n++;
@@ -239,6 +253,12 @@ extern "C" kpzb_status kpzb_gram_compute(kpzb_gram* g, int method, int64_t* G, i
         GCU(cudaGetLastError(), "gram_int64_kernel");
         GCU(cudaMemcpyAsync(gv.data(), g->d_g, 64 * 64 * 8, cudaMemcpyDeviceToHost, g->st), "G copy");
         GCU(cudaStreamSynchronize(g->st), "gram sync");
+    } else if (std::max(-g->vmin, g->vmax) <= GRAM_LOW_RANGE) {
+        // one int8 limb holds every value (surfaces of W < 20 or so): 64 snapshots of 16384^2 take
+        // a third of the three-limb kernel's time
+        kpzb_status st = gram_low_run(geo, g->N, g->sm_count, std::max(-g->vmin, g->vmax), g->d_g, g->tc.d_err,
+                                      gv.data(), g->st);
+        if (st != KPZB_OK) return st;
     } else {
         std::vector<int64_t> gl(192 * 192);
         kpzb_status st = gram_tc_run(&g->tc, geo, g->N, gl.data(), g->st);

@@ -1,8 +1,14 @@
 // gram_slope.cuh -- heights of stored slope snapshots, rebuilt on the fly for the correlator Gram.
 //
-// A snapshot is kept as the two X-slope quadrants of its ENC_CBBIT lattice (Q words each: the
-// X quadrant of sublattice 0, then of sublattice 1; kpz/systemSize.h:143-165) plus, per row y,
-// two int32: b(y) = Hs(y) - c and z(y) = h(0, y) - c, where Hs(y) is the height the reference's
+// A snapshot is kept as the two X-slope quadrants of its ENC_CBBIT lattice (Q words each, the X
+// quadrants of sublattices 0 and 1; kpz/systemSize.h:143-165), 128-site tile by tile: the 16 bytes
+// of tile t -- words 2t and 2t + 1 of sublattice 0's quadrant, then of sublattice 1's -- lie beside
+// those of the other snapshots, at (t * smax + s) * 16.  A warp whose lanes walk 32 snapshots then
+// reads 512 contiguous bytes per tile; from quadrants stored one after the other (64 MiB apart at
+// 16384^2) its lanes touched 128 pages and used 8 bytes of every 32-byte sector: the pipeline of
+// gram_tc.cu with a quarter of its MMAs took 8.2 ms for 64 snapshots that way and 6.6 ms from
+// tiles.  Plus, per row y, two int32:
+//   b(y) = Hs(y) - c and z(y) = h(0, y) - c, where Hs(y) is the height the reference's
 // path walk (kpz/correlator.cpp:47-96) carries into row y before x = 1, h(0, y) the height it
 // gives site x = 0 at the row's end, and c the snapshot's integer mean shift.  Along a row the
 // walk adds 2 s_x(x, y) - 1 for x = 1, 2, ...:
@@ -20,13 +26,20 @@ namespace kpzb {
 constexpr int GS_TILE = 128;  // sites per K tile
 
 struct SlopeSnapGeom {
-    const uint32_t* snap;  // [n][2][Q] X-slope quadrants
+    const uint32_t* snap;  // [Q / 2][smax][2][2] X-slope words: tile, snapshot, sublattice, word
     const int2* rows;      // [n][rows] {b(y), z(y)}
     uint64_t Q;            // words per quadrant
     uint64_t nrows;        // rows of the lattice (2^ly)
     int lx;                // log2 row length
+    int smax;              // snapshots the store has room for
     int n;                 // snapshots present (lanes of absent snapshots produce zeros)
 };
+
+// The four words of tile t of snapshot s.
+__device__ __forceinline__ const uint4* slope_tile(const SlopeSnapGeom& g, int s, uint64_t t)
+{
+    return reinterpret_cast<const uint4*>(g.snap) + (t * (uint64_t)g.smax + (uint64_t)s);
+}
 
 // Running state of one lane: its snapshot, quarter, and the count of X-slope bits of its row
 // in [1, x0) before the current tile (identical in the four lanes of a quad).
@@ -63,13 +76,9 @@ __device__ __forceinline__ SlopeQuarterAddr slope_quarter_addr(const SlopeSnapGe
     if (c.s >= g.n) return SlopeQuarterAddr{nullptr, nullptr, nullptr};
     const int tpr_lg = g.lx - 7;  // log2 tiles per row
     const uint64_t y = t >> tpr_lg;
-    const uint32_t x0 = (uint32_t)(t & ((1ull << tpr_lg) - 1)) << 7;
-    const uint64_t Wr = 1ull << (g.lx - 6);
-    const uint64_t w = y * Wr + (x0 >> 6) + (uint64_t)(c.qt >> 1);
-    const uint32_t* base = g.snap + (uint64_t)c.s * 2 * g.Q;
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(slope_tile(g, c.s, t)) + (c.qt >> 1);
     const int se = (int)(y & 1);
-    return SlopeQuarterAddr{base + (uint64_t)se * g.Q + w, base + (uint64_t)(se ^ 1) * g.Q + w,
-                            g.rows + (uint64_t)c.s * g.nrows + y};
+    return SlopeQuarterAddr{words + 2 * se, words + 2 * (se ^ 1), g.rows + (uint64_t)c.s * g.nrows + y};
 }
 
 __device__ __forceinline__ SlopeQuarter slope_quarter_load(const SlopeSnapGeom& g, const SlopeCursor& c, uint64_t t)
@@ -89,12 +98,16 @@ __device__ __forceinline__ int32_t slope_row_prefix(const SlopeSnapGeom& g, cons
     const uint32_t x0 = (uint32_t)(t & ((1ull << tpr_lg) - 1)) << 7;
     int32_t cnt = 0;
     if (c.s < g.n) {
-        const uint64_t Wr = 1ull << (g.lx - 6);
-        const uint32_t* base = g.snap + (uint64_t)c.s * 2 * g.Q + y * Wr;
-        for (uint32_t j = (uint32_t)c.qt; j < (x0 >> 6); j += 4)
-            cnt += __popc(__ldg(base + j)) + __popc(__ldg(base + g.Q + j));
+        const uint64_t t0 = y << tpr_lg;
+        for (uint32_t j = (uint32_t)c.qt; j < (x0 >> 7); j += 4) {
+            const uint4 v = __ldg(slope_tile(g, c.s, t0 + j));
+            cnt += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+        }
         // site x = 0 (sublattice y & 1, word 0, bit 0) is not part of the walk's running sum
-        if (c.qt == 0 && x0 > 0) cnt -= (int32_t)(__ldg(base + (y & 1) * g.Q) & 1u);
+        if (c.qt == 0 && x0 > 0) {
+            const uint4 v = __ldg(slope_tile(g, c.s, t0));
+            cnt -= (int32_t)((y & 1 ? v.z : v.x) & 1u);
+        }
     }
     cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, 1);
     cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, 2);

@@ -23,10 +23,9 @@
 #include <algorithm>
 #include <cstring>
 
-#include "gram_slope.cuh"
+#include "gram_mma.cuh"
 #include "kpzb_api_internal.h"
 #include "kpzb_gram.h"
-#include "scabit_band.cuh"
 
 namespace kpzb {
 
@@ -41,41 +40,6 @@ constexpr int TC_THREADS = (TC_PROD_WARP0 + TC_PROD_WARPS) * 32;
 constexpr int TC_COLS = 256;                      // TMEM columns: D1 0..191, D2 192..255
 constexpr int TC_LUT = 256;                       // 8-site slope patterns
 constexpr int TC_SMEM = TC_STAGES * TC_STAGE + TC_LUT * 8 + 1024;
-constexpr uint64_t TC_WAIT_NS = 4000000000ull;    // bound of every mbarrier wait (4 s)
-
-// UMMA instruction descriptor, kind::i8: S32 accumulate (bits 4-5 = 2), signed A and B
-// (bits 7-9, 10-12 = 1), both K-major, N>>3 at bit 17, M>>4 at bit 24.
-__host__ __device__ constexpr uint32_t idesc_i8(int M, int N)
-{
-    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-// Shared-memory descriptor of a K-major SWIZZLE_128B operand: rows of 128 bytes, 8-row
-// groups 1024 bytes apart (SBO), LBO 16 bytes, descriptor version 1, layout type 2.
-__device__ __forceinline__ uint64_t sdesc_sw128(uint32_t saddr)
-{
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-           (2ull << 61);
-}
-
-__device__ __forceinline__ uint64_t global_ns()
-{
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// waits for the phase with the given parity; false after TC_WAIT_NS of global time
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity)
-{
-    if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = global_ns();
-    for (;;) {
-        for (int k = 0; k < 64; ++k)
-            if (mbar_try_wait(bar, parity)) return true;
-        if (global_ns() - t0 > TC_WAIT_NS) return false;
-    }
-}
 
 // four values' low bytes, first in the lowest byte
 __device__ __forceinline__ uint32_t pack4(int32_t a, int32_t b, int32_t c, int32_t d)
@@ -88,40 +52,6 @@ __device__ __forceinline__ uint32_t pack4(int32_t a, int32_t b, int32_t c, int32
 __device__ __forceinline__ void put_chunk(uint8_t* stage, int r, int chunk, uint4 v)
 {
     *reinterpret_cast<uint4*>(stage + r * TC_KT + ((chunk ^ (r & 7)) << 4)) = v;
-}
-
-__device__ __forceinline__ void umma_i8(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(dtmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
-}
-
-// Count of X-slope bits of row y in [1, x0) of one snapshot, by one thread (the running count a
-// producer lane starts from when its run of tiles begins inside a row).
-__device__ __forceinline__ int32_t slope_count_before(const SlopeSnapGeom& g, int s, uint64_t y, uint32_t x0)
-{
-    const uint64_t Wr = 1ull << (g.lx - 6);
-    const uint32_t* base = g.snap + (uint64_t)s * 2 * g.Q + y * Wr;
-    int32_t cnt = 0;
-    for (uint32_t j = 0; j < (x0 >> 6); j += 2) {
-        const uint2 a = __ldg(reinterpret_cast<const uint2*>(base + j));
-        const uint2 b = __ldg(reinterpret_cast<const uint2*>(base + g.Q + j));
-        cnt += __popc(a.x) + __popc(a.y) + __popc(b.x) + __popc(b.y);
-    }
-    // site x = 0 (sublattice y & 1, word 0, bit 0) closes the row: not part of the running count
-    if (x0 > 0) cnt -= (int32_t)(__ldg(base + (y & 1) * g.Q) & 1u);
-    return cnt;
 }
 
 // One snapshot's 16 values of K chunk c (sites 16 c .. 16 c + 15 of the tile) by the walk, from
@@ -203,25 +133,19 @@ gram_tc_kernel(const SlopeSnapGeom g, uint64_t nkt, long long* __restrict__ part
         const uint64_t tmask = (1ull << tpr_lg) - 1;
         // lane l: snapshots l and l + 32
         bool pres[2];
-        const uint32_t* qb[2];
         const int2* rb[2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const int s = lane + 32 * k;
             pres[k] = s < g.n;
-            qb[k] = g.snap + (uint64_t)s * 2 * g.Q;
             rb[k] = g.rows + (uint64_t)s * g.nrows;
         }
-        // the next tile's words: [snapshot k][X quadrant], words 2t and 2t + 1
-        uint2 nx[2][2];
+        // the next tile's words of snapshot k: two of sublattice 0's X quadrant, two of sublattice 1's
+        uint4 nx[2];
         auto load = [&](uint64_t t) {
 #pragma unroll
             for (int k = 0; k < 2; ++k)
-#pragma unroll
-                for (int q = 0; q < 2; ++q)
-                    nx[k][q] = (pres[k] && t < cb1)
-                                   ? __ldg(reinterpret_cast<const uint2*>(qb[k] + (uint64_t)q * g.Q + 2 * t))
-                                   : make_uint2(0u, 0u);
+                nx[k] = (pres[k] && t < cb1) ? __ldg(slope_tile(g, lane + 32 * k, t)) : make_uint4(0u, 0u, 0u, 0u);
         };
         load(cb0);
         int32_t B[2] = {0, 0}, z[2] = {0, 0};  // running value before the tile; v(0, y)
@@ -232,8 +156,8 @@ gram_tc_kernel(const SlopeSnapGeom g, uint64_t nkt, long long* __restrict__ part
             uint2 w[2][2];
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                w[k][0] = nx[k][0];
-                w[k][1] = nx[k][1];
+                w[k][0] = make_uint2(nx[k].x, nx[k].y);
+                w[k][1] = make_uint2(nx[k].z, nx[k].w);
             }
             load(t + 1);
             const uint64_t y = t >> tpr_lg;

@@ -23,4 +23,10 @@ void gram_tc_free(GramTC* tc);
 // host out[192*192].
 kpzb_status gram_tc_run(GramTC* tc, const SlopeSnapGeom& g, uint64_t N, int64_t* out, cudaStream_t st);
 
+// The Gram of snapshots with |v| = |h - c| <= range <= GRAM_LOW_RANGE (gram_low.cu); d_g: 64 x 64
+// int64 scratch, out its host copy (upper triangle).
+constexpr int64_t GRAM_LOW_RANGE = 126;
+kpzb_status gram_low_run(const SlopeSnapGeom& g, uint64_t N, int sm_count, int64_t range, unsigned long long* d_g,
+                         unsigned int* d_err, int64_t* out, cudaStream_t st);
+
 }  // namespace kpzb
