@@ -56,7 +56,7 @@ enum DtScheme {
     DT_SCHEME_DB4 = 5
 };
 struct DtState {
-    int grid = 0;
+    int sm_count = 148;
     bool ready = false;
     int scheme = DT_SCHEME_DBSH;  // inner decomposition of a block (the reference's default)
 };
