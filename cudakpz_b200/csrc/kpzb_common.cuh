@@ -82,7 +82,7 @@ __host__ __device__ inline Thresh make_thresh(uint64_t T)
 // and a plane costs eight rounds instead of ten.  A round's two 32 x 32 -> 64 bit products take 4.25
 // cycles each per warp and scheduler, twice a logic operation, so rounds are what a plane is
 // made of.  With the comparison below: (0.95,0.05) at 8192^2 49 -> 42 us per MCS, binary disorder at
-// 4096 x 2048 20 -> 15.6 us (a warp runs as many planes as its slowest lane, 12.6 of a mean 7.5).
+// 4096 x 2048 20 -> 15.6 us.
 struct PlanePart {
     uint32_t x, z, w;
 };
@@ -140,12 +140,15 @@ struct PlaneMaker {
 // six, and selecting each kind's bits two more).  Planes are fetched while a site is undecided,
 // the first four -- a group has about 64 candidates -- without asking.  TB: threshold bit words
 // of plane k; DROP: sites whose threshold has no 1 bit left below plane k (u < T is then false).
-template <class Planes, class TB, class DROP>
+// WARP: all 32 lanes call together, with sixteen words of shared memory per warp in `slot`.  A warp
+// runs until its slowest lane is done, 12.6 planes at (0.95,0.05) where a lane needs 7.5; so once
+// at most half (a quarter) of the lanes have sites left, two (four) lanes compute two (four) planes
+// of each such group at a time: (0.95,0.05) 42 -> 38.5 us per MCS at 8192^2, 138 -> 121 at 16384^2.
+template <bool WARP, class Planes, class TB, class DROP>
 __device__ __forceinline__ uint4 decide_planes(uint4 eq, uint4 flip, int kmax, Key key, const GroupPart& g,
-                                               const Planes& planes, const TB& tb, const DROP& drop)
+                                               const Planes& planes, const TB& tb, const DROP& drop, uint32_t* slot)
 {
-    auto plane = [&](int k) {
-        const uint4 r = philox_plane(g, planes.at(k), key);
+    auto apply = [&](int k, const uint4& r) {
         const uint4 b = tb(k);
         flip.x = (eq.x & b.x) | (~eq.x & flip.x);
         flip.y = (eq.y & b.y) | (~eq.y & flip.y);
@@ -157,21 +160,49 @@ __device__ __forceinline__ uint4 decide_planes(uint4 eq, uint4 flip, int kmax, K
         eq.w &= ~(b.w ^ r.w);
         drop(k, eq, flip);
     };
+    auto plane = [&](int k) { apply(k, philox_plane(g, planes.at(k), key)); };
     int k = 0;
     if (kmax >= 4) {
 #pragma unroll
         for (; k < 4; ++k) plane(k);
     }
-    for (; k < kmax && (eq.x | eq.y | eq.z | eq.w); ++k) plane(k);
+    if constexpr (WARP) {
+        const int lane = (int)(threadIdx.x + threadIdx.y * blockDim.x) & 31;
+        while (k < kmax) {
+            const bool left = (eq.x | eq.y | eq.z | eq.w) != 0u;
+            const uint32_t act = __ballot_sync(0xffffffffu, left);
+            if (!act) break;
+            const int n = __popc(act);
+            if (n > 16) {
+                plane(k++);
+                continue;
+            }
+            const int lg = n > 8 ? 1 : 2, rank = __popc(act & ((1u << lane) - 1u));
+            if (left) slot[rank] = (uint32_t)lane;
+            __syncwarp();
+            const int src = (int)slot[lane >> lg] & 31;  // entries past n: any lane, their planes go unused
+            const GroupPart h{__shfl_sync(0xffffffffu, g.a, src), __shfl_sync(0xffffffffu, g.b, src),
+                              __shfl_sync(0xffffffffu, g.c, src)};
+            const uint4 r = philox_plane(h, planes.at(min(k + (lane & ((1 << lg) - 1)), 31)), key);
+            __syncwarp();
+            for (int j = 0; j < 1 << lg && k < kmax; ++j, ++k) {
+                const int from = (rank << lg) + j;
+                apply(k, make_uint4(__shfl_sync(0xffffffffu, r.x, from), __shfl_sync(0xffffffffu, r.y, from),
+                                    __shfl_sync(0xffffffffu, r.z, from), __shfl_sync(0xffffffffu, r.w, from)));
+            }
+        }
+    } else {
+        for (; k < kmax && (eq.x | eq.y | eq.z | eq.w); ++k) plane(k);
+    }
     // u equal to T in every plane: not below it
     return make_uint4(flip.x & ~eq.x, flip.y & ~eq.y, flip.z & ~eq.z, flip.w & ~eq.w);
 }
 
 // Four-word decision for the 128 sites of one Philox group (qgroup = qword >> 2).
 // cp: local-minimum candidates, cq: local-maximum candidates. Returns the flip mask.
-template <class Planes>
+template <bool WARP = false, class Planes>
 __device__ __forceinline__ uint4 decide4(uint4 cp, uint4 cq, Thresh tp, Thresh tq, Key key, uint32_t qgroup,
-                                         const Planes& planes, uint32_t stream)
+                                         const Planes& planes, uint32_t stream, uint32_t* slot = nullptr)
 {
     const uint32_t ap = tp.always ? 0xFFFFFFFFu : 0u, aq = tq.always ? 0xFFFFFFFFu : 0u;
     const uint32_t hp = tp.planes ? 0xFFFFFFFFu : 0u, hq = tq.planes ? 0xFFFFFFFFu : 0u;
@@ -199,7 +230,8 @@ __device__ __forceinline__ uint4 decide4(uint4 cp, uint4 cq, Thresh tp, Thresh t
         if (k + 1 == tp.planes) out(0u, 0xFFFFFFFFu);
         if (k + 1 == tq.planes) out(0xFFFFFFFFu, 0u);
     };
-    return decide_planes(eq, flip, max(tp.planes, tq.planes), key, group_part(qgroup, stream, key), planes, tb, drop);
+    return decide_planes<WARP>(eq, flip, max(tp.planes, tq.planes), key, group_part(qgroup, stream, key), planes, tb,
+                               drop, slot);
 }
 
 // Decision modes, chosen once per launch from the two thresholds:
@@ -277,7 +309,8 @@ __device__ __forceinline__ uint32_t dis_word(uint32_t cp, uint32_t cq, uint32_t 
 
 template <class Planes>
 __device__ __forceinline__ uint4 decide4_dis(uint4 cp, uint4 cq, uint4 d0, uint4 d1, const DisorderRates& dr,
-                                             Key key, uint32_t qgroup, const Planes& planes, uint32_t stream)
+                                             Key key, uint32_t qgroup, const Planes& planes, uint32_t stream,
+                                             uint32_t* slot)
 {
     uint32_t ap[4], aq[4], hp[4], hq[4];
     for (int c = 0; c < 4; ++c) {
@@ -324,7 +357,7 @@ __device__ __forceinline__ uint4 decide4_dis(uint4 cp, uint4 cq, uint4 d0, uint4
         e.z &= keep.z;
         e.w &= keep.w;
     };
-    return decide_planes(eq, flip, dr.planes, key, group_part(qgroup, stream, key), planes, tb, drop);
+    return decide_planes<true>(eq, flip, dr.planes, key, group_part(qgroup, stream, key), planes, tb, drop, slot);
 }
 
 __device__ __forceinline__ uint4 operator^(uint4 a, uint4 b)

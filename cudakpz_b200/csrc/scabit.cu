@@ -41,9 +41,11 @@ scabit_half_kernel(uint32_t* __restrict__ sys, int lx, int ly, int sigma, uint32
 {
     __shared__ uint32_t nxt_s[SCABIT_THREADS];
     __shared__ uint32_t carry_s[2][SCABIT_THREADS];
+    __shared__ uint32_t slot_s[SCABIT_THREADS / 32][16];
 
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int lin = ty * TX + tx;
+    [[maybe_unused]] uint32_t* slot = slot_s[lin >> 5];
     const uint64_t Wr = 1ull << (lx - 6);
     const uint64_t Q = 1ull << (lx + ly - 6);
     const uint64_t rows = 1ull << ly;
@@ -96,9 +98,9 @@ scabit_half_kernel(uint32_t* __restrict__ sys, int lx, int ly, int sigma, uint32
             if constexpr (DIS) {
                 const uint4 d0 = *reinterpret_cast<const uint4*>(dis + bthisX + roff + wi);
                 const uint4 d1 = *reinterpret_cast<const uint4*>(dis + bthisY + roff + wi);
-                m = decide4_dis(cp, cq, d0, d1, dr, key, (uint32_t)((roff + wi) >> 2), planes, stream);
+                m = decide4_dis(cp, cq, d0, d1, dr, key, (uint32_t)((roff + wi) >> 2), planes, stream, slot);
             } else if constexpr (GENERAL) {
-                m = decide4(cp, cq, tp, tq, key, (uint32_t)((roff + wi) >> 2), planes, stream);
+                m = decide4<true>(cp, cq, tp, tq, key, (uint32_t)((roff + wi) >> 2), planes, stream, slot);
             } else {
                 m = decide4_mode(dec_mode(tp, tq), cp, cq, tp, tq, key, (uint32_t)((roff + wi) >> 2), step,
                                  stream);
