@@ -66,6 +66,10 @@ struct kpzb_handle {
     int fusion = 0;
     bool count = false;
     unsigned long long* d_counters = nullptr;
+    // Whether a kernel with a bounded wait has been enqueued since the last join, which then reads
+    // the flag it may have raised (that copy takes 8 us of every other call); `waits_captured`: in a
+    // graph, whose replays no call here sees.
+    bool waits = false, waits_captured = false;
     // quenched disorder: rate-class words (ENC_LOCAL for DT, ENC_CBBIT form for SCA/SCABit)
     // and the rates of classes 0..3 (class 0 = p, q)
     uint32_t* d_dis = nullptr;
@@ -339,6 +343,7 @@ static kpzb_status resolve_plan_raw(kpzb_handle* h, Plan* plan)
         *plan = default_plan(h->lx, h->ly, Tp, Tq, h->sm_count);
         return KPZB_OK;
     }
+    h->waits = true;
     KPZB_CU(tune_plan(h->d_sys, h->lx, h->ly, h->seed, h->stream_id, Tp, Tq, h->sm_count,
                       reinterpret_cast<unsigned int*>(h->d_counters + 2), h->st, plan),
             "autotune");
@@ -374,6 +379,7 @@ extern "C" kpzb_status kpzb_autotune(kpzb_handle* h, int* mcs_per_pass, int* cta
     KPZB_CHECK_H(h);
     if (h->rs()) return fail(KPZB_EUNSUPPORTED, "the tuner covers SCA/SCABit passes");
     Plan p;
+    h->waits = true;
     KPZB_CU(tune_plan(h->d_sys, h->lx, h->ly, h->seed, h->stream_id, thresh_of(h->p), thresh_of(h->q),
                       h->sm_count, reinterpret_cast<unsigned int*>(h->d_counters + 2), h->st, &p),
             "autotune");
@@ -381,6 +387,14 @@ extern "C" kpzb_status kpzb_autotune(kpzb_handle* h, int* mcs_per_pass, int* cta
     if (ctas_per_sm) *ctas_per_sm = p.cps;
     if (ms_per_mcs) *ms_per_mcs = p.ms_per_mcs;
     return KPZB_OK;
+}
+
+// A kernel with a bounded wait is about to be enqueued.
+static void mark_wait(kpzb_handle* h)
+{
+    h->waits = true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) h->waits_captured = true;
 }
 
 // Whether the left-over MCS of a call may go through the second buffer: not while the caller
@@ -421,6 +435,7 @@ static kpzb_status enqueue_sca(kpzb_handle* h, int n)
             done += k;
         }
     } else if (k > 1 && plan.kind == PASS_WAVE && ws.ok) {
+        mark_wait(h);
         kpzb_status s = ensure_tmp(h);
         if (s != KPZB_OK) return s;
         while (n - done >= k) {
@@ -434,6 +449,7 @@ static kpzb_status enqueue_sca(kpzb_handle* h, int n)
     } else if (k > 1 && plan.kind == PASS_STREAM) {
         const StreamShape ss = scabit_stream_shape(h->lx, h->ly, k, h->sm_count, plan.cps ? plan.cps : 1);
         if (ss.ok) {
+            mark_wait(h);
             kpzb_status s = ensure_tmp(h);
             if (s != KPZB_OK) return s;
             while (n - done >= k) {
@@ -448,6 +464,7 @@ static kpzb_status enqueue_sca(kpzb_handle* h, int n)
     } else if (k > 1) {
         FusedShape fs = scabit_fused_shape_cps(h->lx, h->ly, k, plan.cps, 0);
         if (fs.ok) {
+            mark_wait(h);
             kpzb_status s = ensure_tmp(h);
             if (s != KPZB_OK) return s;
             while (n - done >= k) {
@@ -483,6 +500,7 @@ static kpzb_status enqueue_sca(kpzb_handle* h, int n)
     } else if (spare && plan.kind == PASS_BAND && n - done < k) {
         const FusedShape rest = scabit_fused_shape_cps(h->lx, h->ly, n - done, plan.cps, 0);
         if (rest.ok) {
+            mark_wait(h);
             KPZB_CU(scabit_fused(h->d_sys, h->d_tmp, h->lx, h->ly, (uint32_t)(h->tdev + done), h->seed, h->stream_id,
                                  Tp, Tq, rest, cnt, reinterpret_cast<unsigned int*>(h->d_counters + 2), h->st),
                     "scabit_fused");
@@ -561,10 +579,11 @@ extern "C" kpzb_status kpzb_join(kpzb_handle* h)
 {
     KPZB_CHECK_H(h);
     unsigned int flag = 0;
-    KPZB_CU(cudaMemcpyAsync(&flag, h->d_counters + 2, sizeof flag, cudaMemcpyDeviceToHost, h->st),
-            "join flag");
+    if (h->waits || h->waits_captured)
+        KPZB_CU(cudaMemcpyAsync(&flag, h->d_counters + 2, sizeof flag, cudaMemcpyDeviceToHost, h->st), "join flag");
     KPZB_CU(cudaStreamSynchronize(h->st), "join");
     KPZB_CU(cudaGetLastError(), "join");
+    h->waits = false;
     if (flag) {
         cudaMemsetAsync(h->d_counters + 2, 0, sizeof(unsigned long long), h->st);
         cudaStreamSynchronize(h->st);
