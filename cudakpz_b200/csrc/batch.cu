@@ -122,6 +122,7 @@ struct kpzb_batch {
     bool planned = false;        // k and cps set by the caller or the tuner (else tuned on first MCS)
     cudaGraphExec_t graph = nullptr;
     AnalysisScratch an{};
+    unsigned char* d_rec = nullptr;  // roughness records of all replicas
     int max_ly = 0;
 };
 
@@ -278,6 +279,7 @@ extern "C" kpzb_status kpzb_batch_destroy(kpzb_batch* b)
     cudaFree(b->d_reps);
     cudaFree(b->d_items);
     cudaFree(b->d_state);
+    cudaFree(b->d_rec);
     if (b->an.rowinfo) analysis_free(&b->an);
     if (b->st) cudaStreamDestroy(b->st);
     delete b;
@@ -548,12 +550,25 @@ extern "C" kpzb_status kpzb_batch_roughness(kpzb_batch* b, double* w2)
 {
     BCHECK(b);
     if (!w2) return fail(KPZB_EINVAL, "null output");
+    // every replica's reduction behind the other, one copy of the records at the end (a copy and a
+    // wait per replica took longer than the reductions)
+    const size_t rb = analysis_record_bytes();
+    cudaError_t e;
+    if (!b->d_rec && (e = cudaMalloc(&b->d_rec, rb * (size_t)b->n)) != cudaSuccess)
+        return cuda_fail(e, "cudaMalloc(batch records)");
     for (int i = 0; i < b->n; ++i) {
         const RepDesc& r = b->reps[i];
-        MomentsOut m;
-        const cudaError_t e = analysis_moments(r.buf[b->parity], nullptr, r.lx, r.ly, &b->an, &m, b->st);
+        e = analysis_moments_record(r.buf[b->parity], nullptr, r.lx, r.ly, &b->an, b->d_rec + (size_t)i * rb, b->st);
         if (e != cudaSuccess) return cuda_fail(e, "batch roughness");
-        const long double N = (long double)((uint64_t)1 << (2 * r.lx));
+    }
+    std::vector<unsigned char> host(rb * (size_t)b->n);
+    if ((e = cudaMemcpyAsync(host.data(), b->d_rec, host.size(), cudaMemcpyDeviceToHost, b->st)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(b->st)) != cudaSuccess)
+        return cuda_fail(e, "batch roughness");
+    for (int i = 0; i < b->n; ++i) {
+        MomentsOut m;
+        analysis_decode_record(host.data() + (size_t)i * rb, &m);
+        const long double N = (long double)((uint64_t)1 << (2 * b->reps[i].lx));
         const long double h1 = (long double)m.s1 / N, h2 = (long double)m.s2 / N;
         w2[i] = (double)(h2 - h1 * h1);
     }
