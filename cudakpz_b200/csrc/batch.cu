@@ -30,8 +30,9 @@ namespace kpzb {
 constexpr int BATCH_THREADS = 512;  // threads of a CTA at one CTA per SM; 256 at two or three
 constexpr size_t BATCH_SMEM = 227 * 1024 - 1024;
 
-// shared memory of one CTA at `cps` CTAs per SM (the SM's 228 KB split, 1 KB each reserved)
-inline size_t batch_smem(int cps) { return cps <= 1 ? BATCH_SMEM : ((228 * 1024) / (size_t)cps - 1024) & ~(size_t)127; }
+// shared memory of one CTA at `cps` CTAs per SM (the SM's 228 KB split, less 1 KB each that the
+// system reserves and 1 KB for static shared memory)
+inline size_t batch_smem(int cps) { return cps <= 1 ? BATCH_SMEM : ((228 * 1024) / (size_t)cps - 2048) & ~(size_t)127; }
 inline int batch_threads(int cps) { return cps <= 1 ? BATCH_THREADS : 256; }
 
 struct RepDesc {

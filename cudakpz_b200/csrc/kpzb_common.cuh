@@ -140,13 +140,13 @@ struct PlaneMaker {
 // six, and selecting each kind's bits two more).  Planes are fetched while a site is undecided,
 // the first four -- a group has about 64 candidates -- without asking.  TB: threshold bit words
 // of plane k; DROP: sites whose threshold has no 1 bit left below plane k (u < T is then false).
-// WARP: all 32 lanes call together, with sixteen words of shared memory per warp in `slot`.  A warp
+// WARP: all 32 lanes call together, with sixteen bytes of shared memory per warp in `slot`.  A warp
 // runs until its slowest lane is done, 12.6 planes at (0.95,0.05) where a lane needs 7.5; so once
 // at most half (a quarter) of the lanes have sites left, two (four) lanes compute two (four) planes
 // of each such group at a time: (0.95,0.05) 42 -> 38.5 us per MCS at 8192^2, 138 -> 121 at 16384^2.
 template <bool WARP, class Planes, class TB, class DROP>
 __device__ __forceinline__ uint4 decide_planes(uint4 eq, uint4 flip, int kmax, Key key, const GroupPart& g,
-                                               const Planes& planes, const TB& tb, const DROP& drop, uint32_t* slot)
+                                               const Planes& planes, const TB& tb, const DROP& drop, uint8_t* slot)
 {
     auto apply = [&](int k, const uint4& r) {
         const uint4 b = tb(k);
@@ -166,7 +166,7 @@ __device__ __forceinline__ uint4 decide_planes(uint4 eq, uint4 flip, int kmax, K
 #pragma unroll
         for (; k < 4; ++k) plane(k);
     }
-    if constexpr (WARP) {
+    if (WARP && kmax > 4) {
         const int lane = (int)(threadIdx.x + threadIdx.y * blockDim.x) & 31;
         while (k < kmax) {
             const bool left = (eq.x | eq.y | eq.z | eq.w) != 0u;
@@ -178,7 +178,7 @@ __device__ __forceinline__ uint4 decide_planes(uint4 eq, uint4 flip, int kmax, K
                 continue;
             }
             const int lg = n > 8 ? 1 : 2, rank = __popc(act & ((1u << lane) - 1u));
-            if (left) slot[rank] = (uint32_t)lane;
+            if (left) slot[rank] = (uint8_t)lane;
             __syncwarp();
             const int src = (int)slot[lane >> lg] & 31;  // entries past n: any lane, their planes go unused
             const GroupPart h{__shfl_sync(0xffffffffu, g.a, src), __shfl_sync(0xffffffffu, g.b, src),
@@ -202,7 +202,7 @@ __device__ __forceinline__ uint4 decide_planes(uint4 eq, uint4 flip, int kmax, K
 // cp: local-minimum candidates, cq: local-maximum candidates. Returns the flip mask.
 template <bool WARP = false, class Planes>
 __device__ __forceinline__ uint4 decide4(uint4 cp, uint4 cq, Thresh tp, Thresh tq, Key key, uint32_t qgroup,
-                                         const Planes& planes, uint32_t stream, uint32_t* slot = nullptr)
+                                         const Planes& planes, uint32_t stream, uint8_t* slot = nullptr)
 {
     const uint32_t ap = tp.always ? 0xFFFFFFFFu : 0u, aq = tq.always ? 0xFFFFFFFFu : 0u;
     const uint32_t hp = tp.planes ? 0xFFFFFFFFu : 0u, hq = tq.planes ? 0xFFFFFFFFu : 0u;
@@ -227,18 +227,69 @@ __device__ __forceinline__ uint4 decide4(uint4 cp, uint4 cq, Thresh tp, Thresh t
             one(cq.z, e.z, f.z);
             one(cq.w, e.w, f.w);
         };
-        if (k + 1 == tp.planes) out(0u, 0xFFFFFFFFu);
-        if (k + 1 == tq.planes) out(0xFFFFFFFFu, 0u);
+        // (at the last plane of all, what is left is dropped anyway)
+        if (k + 1 == tp.planes && tp.planes < tq.planes) out(0u, 0xFFFFFFFFu);
+        if (k + 1 == tq.planes && tq.planes < tp.planes) out(0xFFFFFFFFu, 0u);
     };
     return decide_planes<WARP>(eq, flip, max(tp.planes, tq.planes), key, group_part(qgroup, stream, key), planes, tb,
                                drop, slot);
+}
+
+// The same decision for rates of at most four planes (DEC_FEW): whole Philox calls and a mask per
+// kind of candidate.  With two planes there is little to share and lanes hardly differ:
+// (0.75,0.25) at 8192^2 in band passes takes 15.5 us per MCS this way, 16.3 with decide4.
+__device__ __forceinline__ uint4 decide4_few(uint4 cp, uint4 cq, Thresh tp, Thresh tq, Key key,
+                                         uint32_t qgroup, uint32_t step, uint32_t stream)
+{
+    uint4 ltp, eqp, ltq, eqq;
+    if (tp.always) {
+        ltp = cp;
+        eqp = make_uint4(0, 0, 0, 0);
+    } else {
+        ltp = make_uint4(0, 0, 0, 0);
+        eqp = tp.planes ? cp : make_uint4(0, 0, 0, 0);
+    }
+    if (tq.always) {
+        ltq = cq;
+        eqq = make_uint4(0, 0, 0, 0);
+    } else {
+        ltq = make_uint4(0, 0, 0, 0);
+        eqq = tq.planes ? cq : make_uint4(0, 0, 0, 0);
+    }
+    const int kmax = max(tp.planes, tq.planes);
+    for (int k = 0; k < kmax; ++k) {
+        const uint32_t any = eqp.x | eqp.y | eqp.z | eqp.w | eqq.x | eqq.y | eqq.z | eqq.w;
+        if (!any) break;
+        const uint4 r = philox4x32_10(make_uint4(qgroup, step, (uint32_t)k | (TAG_SCA << 8), stream), key);
+        const uint32_t bp = (tp.t >> (31 - k)) & 1u;
+        const uint32_t bq = (tq.t >> (31 - k)) & 1u;
+        // bit of T is 1: sites with u-bit 0 are below T (decided), u-bit 1 stay equal.
+        // bit of T is 0: sites with u-bit 1 are above T (drop), u-bit 0 stay equal.
+        if (bp) {
+            ltp.x |= eqp.x & ~r.x; ltp.y |= eqp.y & ~r.y; ltp.z |= eqp.z & ~r.z; ltp.w |= eqp.w & ~r.w;
+            eqp.x &= r.x; eqp.y &= r.y; eqp.z &= r.z; eqp.w &= r.w;
+        } else {
+            eqp.x &= ~r.x; eqp.y &= ~r.y; eqp.z &= ~r.z; eqp.w &= ~r.w;
+        }
+        if (bq) {
+            ltq.x |= eqq.x & ~r.x; ltq.y |= eqq.y & ~r.y; ltq.z |= eqq.z & ~r.z; ltq.w |= eqq.w & ~r.w;
+            eqq.x &= r.x; eqq.y &= r.y; eqq.z &= r.z; eqq.w &= r.w;
+        } else {
+            eqq.x &= ~r.x; eqq.y &= ~r.y; eqq.z &= ~r.z; eqq.w &= ~r.w;
+        }
+        if (k + 1 >= tp.planes) eqp = make_uint4(0, 0, 0, 0);
+        if (k + 1 >= tq.planes) eqq = make_uint4(0, 0, 0, 0);
+    }
+    return make_uint4(ltp.x | ltq.x, ltp.y | ltq.y, ltp.z | ltq.z, ltp.w | ltq.w);
 }
 
 // Decision modes, chosen once per launch from the two thresholds:
 //   DEC_NONE   no random plane can matter (every threshold is 0 or 2^32),
 //   DEC_ONE    at most the MSB plane matters (thresholds in {0, 2^31, 2^32}, e.g. p = 1/2),
 //   DEC_GENERAL anything else (bit-serial loop of decide4).
-enum DecMode { DEC_NONE = 0, DEC_ONE = 1, DEC_GENERAL = 2 };
+//   DEC_FEW    DEC_GENERAL's rates of at most four planes, where a kernel has an instance of its own
+//              for them (decide4_few).
+enum DecMode { DEC_NONE = 0, DEC_ONE = 1, DEC_GENERAL = 2, DEC_FEW = 3 };
 
 __host__ __device__ inline int dec_mode(Thresh tp, Thresh tq)
 {
@@ -247,9 +298,11 @@ __host__ __device__ inline int dec_mode(Thresh tp, Thresh tq)
 }
 
 // decide4 with the cheap modes spelled out; identical results in every mode.
+// slot: sixteen bytes of shared memory per warp where all 32 lanes call together, else nullptr.
+template <bool WARP = false>
 __device__ __forceinline__ uint4 decide4_mode(int mode, uint4 cp, uint4 cq, Thresh tp, Thresh tq,
                                               Key key, uint32_t qgroup, uint32_t step,
-                                              uint32_t stream)
+                                              uint32_t stream, uint8_t* slot = nullptr)
 {
     if (mode == DEC_NONE) {
         const uint32_t ap = tp.always ? 0xFFFFFFFFu : 0u, aq = tq.always ? 0xFFFFFFFFu : 0u;
@@ -268,7 +321,8 @@ __device__ __forceinline__ uint4 decide4_mode(int mode, uint4 cp, uint4 cq, Thre
                           (cp.z & (ap | (hp & ~r.z))) | (cq.z & (aq | (hq & ~r.z))),
                           (cp.w & (ap | (hp & ~r.w))) | (cq.w & (aq | (hq & ~r.w))));
     }
-    return decide4(cp, cq, tp, tq, key, qgroup, PlaneMaker{step, key}, stream);
+    if (mode == DEC_FEW) return decide4_few(cp, cq, tp, tq, key, qgroup, step, stream);
+    return decide4<WARP>(cp, cq, tp, tq, key, qgroup, PlaneMaker{step, key}, stream, slot);
 }
 
 // Quenched disorder (mcsDisorder2SyncRng): every site carries a 2-bit rate class c (bit 0 in
@@ -277,7 +331,7 @@ __device__ __forceinline__ uint4 decide4_mode(int mode, uint4 cp, uint4 cq, Thre
 struct DisorderRates {
     Thresh tp[4], tq[4];
     int planes;            // most planes any of the eight thresholds can need
-    uint32_t last_planes;  // bit k: plane k is the last that one of them can need
+    uint32_t last_planes;  // bit k: plane k is the last that one of them, but not the last of all, can need
 };
 
 inline DisorderRates make_disorder_rates(const uint64_t Tp[4], const uint64_t Tq[4])
@@ -291,6 +345,7 @@ inline DisorderRates make_disorder_rates(const uint64_t Tp[4], const uint64_t Tq
         if (dr.tp[c].planes) dr.last_planes |= 1u << (dr.tp[c].planes - 1);
         if (dr.tq[c].planes) dr.last_planes |= 1u << (dr.tq[c].planes - 1);
     }
+    if (dr.planes) dr.last_planes &= ~(1u << (dr.planes - 1));  // there, what is left is dropped anyway
     return dr;
 }
 
@@ -310,7 +365,7 @@ __device__ __forceinline__ uint32_t dis_word(uint32_t cp, uint32_t cq, uint32_t 
 template <class Planes>
 __device__ __forceinline__ uint4 decide4_dis(uint4 cp, uint4 cq, uint4 d0, uint4 d1, const DisorderRates& dr,
                                              Key key, uint32_t qgroup, const Planes& planes, uint32_t stream,
-                                             uint32_t* slot)
+                                             uint8_t* slot)
 {
     uint32_t ap[4], aq[4], hp[4], hq[4];
     for (int c = 0; c < 4; ++c) {

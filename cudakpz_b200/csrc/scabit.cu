@@ -41,11 +41,11 @@ scabit_half_kernel(uint32_t* __restrict__ sys, int lx, int ly, int sigma, uint32
 {
     __shared__ uint32_t nxt_s[SCABIT_THREADS];
     __shared__ uint32_t carry_s[2][SCABIT_THREADS];
-    __shared__ uint32_t slot_s[SCABIT_THREADS / 32][16];
+    __shared__ uint8_t slot_s[SCABIT_THREADS / 32][16];
 
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int lin = ty * TX + tx;
-    [[maybe_unused]] uint32_t* slot = slot_s[lin >> 5];
+    [[maybe_unused]] uint8_t* slot = slot_s[lin >> 5];
     const uint64_t Wr = 1ull << (lx - 6);
     const uint64_t Q = 1ull << (lx + ly - 6);
     const uint64_t rows = 1ull << ly;
@@ -310,7 +310,7 @@ static cudaError_t launch_fused(const uint32_t* d_src, uint32_t* d_dst, int lx, 
     // the general bit-serial decision keeps 512 threads (its registers do not fit 64)
     auto kern = scabit_fused_kernel<MODE, USEQ, COUNT, FUSED_THREADS>;
     int nt = FUSED_THREADS;
-    if constexpr (MODE != DEC_GENERAL) {
+    if constexpr (MODE == DEC_NONE || MODE == DEC_ONE) {
         if (sh.threads == FUSED_THREADS_WIDE) {
             kern = scabit_fused_kernel<MODE, USEQ, COUNT, FUSED_THREADS_WIDE>;
             nt = FUSED_THREADS_WIDE;
@@ -351,6 +351,7 @@ cudaError_t scabit_fused(const uint32_t* d_src, uint32_t* d_dst, int lx, int ly,
                                            d_err, st)
     if (mode == DEC_NONE) KPZB_FUSED_CASE(DEC_NONE);
     if (mode == DEC_ONE) KPZB_FUSED_CASE(DEC_ONE);
+    if (tp.planes <= 4 && tq.planes <= 4) KPZB_FUSED_CASE(DEC_FEW);
     KPZB_FUSED_CASE(DEC_GENERAL);
 #undef KPZB_FUSED_CASE
 }

@@ -12,6 +12,8 @@
 // kpz/kpzSCABitCores.cu:69-74,139-145.  The one-bit x-carry of shifted rows crosses thread
 // boundaries only in the first word of each 4-word group (shared-memory atomicXor).
 #pragma once
+#include <type_traits>
+
 #include "kpzb_common.cuh"
 
 namespace kpzb {
@@ -114,10 +116,11 @@ __device__ __forceinline__ GroupIn sca_load_group(const uint32_t* pTX, const uin
 
 // Candidate masks and flip mask of one 4-word group from its words (xX: the other-X words as
 // seen by this sublattice's sites, i.e. shifted for shifted rows).
-template <int MODE, bool USEQ>
+template <int MODE, bool USEQ, bool WARP = false>
 __device__ __forceinline__ uint4 sca_decide(const uint4& tX, const uint4& tY, const uint4& xX, const uint4& oY,
                                             int mode_rt, const Thresh& tp, const Thresh& tq, Key key,
-                                            uint32_t qgroup, uint32_t step, uint32_t stream, uint4& cp, uint4& cq)
+                                            uint32_t qgroup, uint32_t step, uint32_t stream, uint4& cp, uint4& cq, bool live = true,
+                                            uint8_t* slot = nullptr)
 {
     cq = make_uint4(0, 0, 0, 0);
     cp.x = ~(tX.x | tY.x) & xX.x & oY.x;
@@ -137,7 +140,8 @@ __device__ __forceinline__ uint4 sca_decide(const uint4& tX, const uint4& tY, co
         return make_uint4((cp.x & ap) | (cq.x & aq), (cp.y & ap) | (cq.y & aq), (cp.z & ap) | (cq.z & aq),
                           (cp.w & ap) | (cq.w & aq));
     }
-    return decide4_mode(MODE < 0 ? mode_rt : MODE, cp, cq, tp, tq, key, qgroup, step, stream);
+    if (WARP && !live) cp = cq = make_uint4(0, 0, 0, 0);
+    return decide4_mode<WARP>(MODE < 0 ? mode_rt : MODE, cp, cq, tp, tq, key, qgroup, step, stream, slot);
 }
 
 // The update of one group from its loaded words.  Within a half-step a group may be loaded
@@ -146,12 +150,13 @@ __device__ __forceinline__ uint4 sca_decide(const uint4& tX, const uint4& tY, co
 // half-step reads or writes, except the next group's first other-X word, whose bit 0 it
 // changes by an atomic XOR -- a bit the owner neither reads (the one-bit right shift drops it)
 // nor stores (it XORs its own mask in atomically).
-template <int MODE, bool USEQ, bool COUNT>
+template <int MODE, bool USEQ, bool COUNT, bool WARP = false>
 __device__ __forceinline__ void sca_update_loaded(const GroupIn& in, uint32_t* pTX, uint32_t* pTY, uint32_t* pOX,
                                                   uint32_t* pOY, uint32_t* nbp, bool shifted, int mode_rt,
                                                   const Thresh& tp, const Thresh& tq, Key key, uint32_t qgroup,
                                                   uint32_t step, uint32_t stream, bool count_row,
-                                                  unsigned long long& ndep, unsigned long long& ndes)
+                                                  unsigned long long& ndep, unsigned long long& ndes,
+                                                  bool live = true, uint8_t* slot = nullptr)
 {
     const uint4 tX = in.tX, tY = in.tY, oX = in.oX, oY = in.oY;
     uint4 xX = oX;
@@ -162,7 +167,9 @@ __device__ __forceinline__ void sca_update_loaded(const GroupIn& in, uint32_t* p
         xX.w = __funnelshift_r(oX.w, in.nb, 1);
     }
     uint4 cp, cq;
-    const uint4 m = sca_decide<MODE, USEQ>(tX, tY, xX, oY, mode_rt, tp, tq, key, qgroup, step, stream, cp, cq);
+    const uint4 m = sca_decide<MODE, USEQ, WARP>(tX, tY, xX, oY, mode_rt, tp, tq, key, qgroup, step, stream, cp, cq,
+                                                 live, slot);
+    if (WARP && !live) return;
     if (COUNT && count_row) {
         ndep += __popc(m.x & cp.x) + __popc(m.y & cp.y) + __popc(m.z & cp.z) + __popc(m.w & cp.w);
         if (USEQ) ndes += __popc(m.x & cq.x) + __popc(m.y & cq.y) + __popc(m.z & cq.z) + __popc(m.w & cq.w);
@@ -190,17 +197,20 @@ __device__ __forceinline__ void sca_update_loaded(const GroupIn& in, uint32_t* p
 // drops the maximum-candidate mask.  The carry crosses groups with shared-memory atomicXor on
 // disjoint bits (bit 0 of the next group's first word; bits 1..31 of this group's), so
 // neighbouring groups of a row may be updated concurrently.
-template <int MODE, bool USEQ, bool COUNT>
+// WARP: all 32 lanes of the warp call together (general rates then share planes, decide_planes), those
+// without a group of their own with live = false and the pointers of some other group.
+template <int MODE, bool USEQ, bool COUNT, bool WARP = false>
 __device__ __forceinline__ void sca_update_group(uint32_t* pTX, uint32_t* pTY, uint32_t* pOX,
                                                  uint32_t* pOY, uint32_t* nbp, bool shifted,
                                                  int mode_rt, const Thresh& tp, const Thresh& tq,
                                                  Key key, uint32_t qgroup, uint32_t step,
                                                  uint32_t stream, bool count_row,
-                                                 unsigned long long& ndep, unsigned long long& ndes)
+                                                 unsigned long long& ndep, unsigned long long& ndes,
+                                                 bool live = true, uint8_t* slot = nullptr)
 {
     const GroupIn in = sca_load_group(pTX, pTY, pOX, pOY, nbp);
-    sca_update_loaded<MODE, USEQ, COUNT>(in, pTX, pTY, pOX, pOY, nbp, shifted, mode_rt, tp, tq, key, qgroup,
-                                         step, stream, count_row, ndep, ndes);
+    sca_update_loaded<MODE, USEQ, COUNT, WARP>(in, pTX, pTY, pOX, pOY, nbp, shifted, mode_rt, tp, tq, key, qgroup,
+                                               step, stream, count_row, ndep, ndes, live, slot);
 }
 
 // Runs one band; returns false (after flagging *err) when the TMA load did not complete in
@@ -261,7 +271,9 @@ __device__ bool scabit_band(uint32_t* smem, const BandCtl& ctl, const BandGeom& 
     // shared-memory offsets are 32-bit (a band is at most 227 KB).  (A warp-per-row variant
     // that passes the x-carry by shuffles removed the atomics and bank conflicts but issued
     // 67 % more instructions and ran 15 % slower at 16384^2; the atomics stay.)
-    const int mode_rt = MODE < 0 ? dec_mode(g.tp, g.tq) : MODE;
+    __shared__ uint8_t slot_s[NT / 32][16];
+    const bool few = g.tp.planes <= 4 && g.tq.planes <= 4;
+    const int mode_rt = MODE < 0 ? (dec_mode(g.tp, g.tq) == DEC_GENERAL && few ? DEC_FEW : dec_mode(g.tp, g.tq)) : MODE;
     const uint32_t wr = (uint32_t)Wr;
     const int gi = (G >= NT) ? (int)threadIdx.x : (int)(threadIdx.x & (G - 1));
     const int rstride = (G >= NT) ? 1 : NT >> lgG;
@@ -278,19 +290,31 @@ __device__ bool scabit_band(uint32_t* smem, const BandCtl& ctl, const BandGeom& 
         uint32_t* SoY = SoX + q32;
         const int ra = g.resident ? 0 : h;
         const int rb = g.resident ? R : R - 1 - h;
-        // wide rows (G > NT): a thread takes several column groups of a row in turn
-        for (int gg = gi; gg < G; gg += NT) {
+        auto update = [&](auto warp_tag, int gg, int lr, bool live) {
+            constexpr bool WARP = decltype(warp_tag)::value;
             const uint32_t w0 = 4u * (uint32_t)gg;
             const uint32_t wnext = (w0 + 4u) & (wr - 1u);
-            for (int lr = ra + rofs; lr < rb; lr += rstride) {
-                const uint32_t gy = ((uint32_t)ylo32 + (uint32_t)lr) & rmask;  // periodic in y
-                const uint32_t ro = (uint32_t)lr * wr;
-                const uint32_t ro1 = g.resident ? (((uint32_t)lr + 1u) & rmask) * wr : ro + wr;
-                sca_update_group<MODE, USEQ, COUNT>(StX + ro + w0, StY + ro + w0, SoX + ro + w0, SoY + ro1 + w0,
-                                                    SoX + ro + wnext, sigma != (int)(gy & 1u), mode_rt, g.tp,
-                                                    g.tq, g.key, (gy << lgG) + (uint32_t)gg, step, g.stream,
-                                                    lr >= H && lr < H + Bc, ndep, ndes);
-            }
+            const uint32_t gy = ((uint32_t)ylo32 + (uint32_t)lr) & rmask;  // periodic in y
+            const uint32_t ro = (uint32_t)lr * wr;
+            const uint32_t ro1 = g.resident ? (((uint32_t)lr + 1u) & rmask) * wr : ro + wr;
+            sca_update_group<MODE, USEQ, COUNT, WARP>(StX + ro + w0, StY + ro + w0, SoX + ro + w0, SoY + ro1 + w0,
+                                                      SoX + ro + wnext, sigma != (int)(gy & 1u), mode_rt, g.tp, g.tq,
+                                                      g.key, (gy << lgG) + (uint32_t)gg, step, g.stream,
+                                                      lr >= H && lr < H + Bc, ndep, ndes, live, slot_s[threadIdx.x >> 5]);
+        };
+        if (MODE == DEC_GENERAL || (MODE < 0 && mode_rt == DEC_GENERAL)) {
+            // every warp stays together: lanes past the last row repeat a row without effect
+            for (int gg = gi; gg < G; gg += NT)
+                for (int l0 = ra; l0 < rb; l0 += rstride) {
+                    const int lr = l0 + rofs;
+                    update(std::true_type{}, gg, lr < rb ? lr : ra, lr < rb);
+                }
+            __syncthreads();
+            continue;
+        }
+        // wide rows (G > NT): a thread takes several column groups of a row in turn
+        for (int gg = gi; gg < G; gg += NT) {
+            for (int lr = ra + rofs; lr < rb; lr += rstride) update(std::false_type{}, gg, lr, true);
         }
         __syncthreads();
     }
