@@ -389,12 +389,20 @@ extern "C" kpzb_status kpzb_autotune(kpzb_handle* h, int* mcs_per_pass, int* cta
     return KPZB_OK;
 }
 
+// Whether the caller captures the handle's stream (or the runtime will not say).
+static bool capturing(const kpzb_handle* h)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->st, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 // A kernel with a bounded wait is about to be enqueued.
 static void mark_wait(kpzb_handle* h)
 {
     h->waits = true;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(h->st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) h->waits_captured = true;
+    if (capturing(h)) h->waits_captured = true;
 }
 
 // Whether the left-over MCS of a call may go through the second buffer: not while the caller
@@ -402,8 +410,7 @@ static void mark_wait(kpzb_handle* h)
 // updating the lattice in place), nor when there is no memory for it.
 static bool spare_buffer(kpzb_handle* h)
 {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(h->st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+    if (capturing(h)) return false;
     if (ensure_tmp(h) == KPZB_OK) return true;
     cudaGetLastError();
     g_err.clear();
