@@ -83,13 +83,26 @@ __device__ __forceinline__ long long cta_exclusive_scan(long long v, long long* 
     return before + incl - v;
 }
 
+__host__ inline bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
+
+// Four words from p on: one 128-bit load, or word by word.
+template <bool WORDS>
+__device__ __forceinline__ uint4 load_words4(const uint32_t* p)
+{
+    if (WORDS) return make_uint4(p[0], p[1], p[2], p[3]);
+    return *reinterpret_cast<const uint4*>(p);
+}
+
 // ---- launch 1: per-row slope counts and row starts within a block of rows ----
 // A CTA takes one block of rows; blockIdx.y picks the lattice (the system, the snapshot).  A warp
 // reads a row's 2 Wr words as 128-bit loads, ordered quarter by quarter and both X quadrants of
 // a quarter together, so that every lane has a load of every step; rows shorter than
-// AN_PART_WORDS take Wr / 2 lanes each.  The scan over blocks is left to each reader, which needs
+// AN_PART_WORDS take Wr / 2 lanes each.  A caller's own lattice may start at any word
+// (kpzb_roughness_noalloc, kpzb_gram_add_device): off a 16-byte boundary the instance WORDS reads
+// the same 16 bytes word by word.  The scan over blocks is left to each reader, which needs
 // no grid-wide step: a scan of all rows by one CTA (a launch of its own, or the last CTA here)
 // took 15 to 27 us at 8192 and 16384 rows, most of both kernels' time.
+template <bool WORDS>
 __global__ void __launch_bounds__(AN_ROW_THREADS)
 row_kernel(const uint32_t* __restrict__ sys0, const uint32_t* __restrict__ sys1, int lx, int ly,
            int4* __restrict__ rowinfo0, int64_t* __restrict__ rowstart0, WalkState* ws)
@@ -108,6 +121,7 @@ row_kernel(const uint32_t* __restrict__ sys0, const uint32_t* __restrict__ sys1,
     const uint64_t yb = (uint64_t)blockIdx.x << lgb, ye = yb + (1ull << lgb);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) ws->ticket = 0u;
     auto count4 = [](uint4 v) { return __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w); };
+    auto load4 = [](const uint32_t* r, uint64_t i) { return load_words4<WORDS>(r + 4 * i); };
     // site (0,y) lies on sublattice y&1, word 0, bit 0
     auto sy0 = [&](uint64_t y) { return (int)(sys[((y & 1) ? 2 * Q : 0) + Q + y * Wr] & 1u); };
     long long carry = 0, lo = 0x7fffffffffffffffll, hi = -0x7fffffffffffffffll;
@@ -123,13 +137,13 @@ row_kernel(const uint32_t* __restrict__ sys0, const uint32_t* __restrict__ sys1,
 #pragma unroll 2
             for (uint64_t y = base + wid; y < end; y += NWARP) {
                 const int s = sy0(y);
-                const uint4* r0 = reinterpret_cast<const uint4*>(sys + y * Wr);
-                const uint4* r1 = reinterpret_cast<const uint4*>(sys + 2 * Q + y * Wr);
+                const uint32_t* r0 = sys + y * Wr;
+                const uint32_t* r1 = sys + 2 * Q + y * Wr;
                 int n[4] = {0, 0, 0, 0};
                 if (qv == 8) {  // a step of the warp covers two quarters
                     uint4 v[2];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) v[h] = (lane & 8 ? r1 : r0)[16 * h + 8 * (lane >> 4) + (lane & 7)];
+                    for (int h = 0; h < 2; ++h) v[h] = load4(lane & 8 ? r1 : r0, 16 * h + 8 * (lane >> 4) + (lane & 7));
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const int c = count4(v[h]);
@@ -140,7 +154,7 @@ row_kernel(const uint32_t* __restrict__ sys0, const uint32_t* __restrict__ sys1,
                     for (uint64_t i = lane; i < 2 * qv; i += 32) {
                         uint4 v[4];
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) v[q] = i >= qv ? r1[q * qv + i - qv] : r0[q * qv + i];
+                        for (int q = 0; q < 4; ++q) v[q] = i >= qv ? load4(r1, q * qv + i - qv) : load4(r0, q * qv + i);
 #pragma unroll
                         for (int q = 0; q < 4; ++q) n[q] += count4(v[q]);
                     }
@@ -156,7 +170,7 @@ row_kernel(const uint32_t* __restrict__ sys0, const uint32_t* __restrict__ sys1,
                 const int j = lane % sw, half = sw / 2;
                 const bool in = y < end;
                 const int s = in ? sy0(y) : 0;
-                int n = in ? count4(reinterpret_cast<const uint4*>(sys + (j >= half ? 2 * Q : 0) + y * Wr)[j % half]) : 0;
+                int n = in ? count4(load4(sys + (j >= half ? 2 * Q : 0) + y * Wr, j % half)) : 0;
                 for (int o = 1; o < sw; o <<= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
                 if (in && j == 0) put(y, 0, 0, 0, n, s);
             }
@@ -686,8 +700,8 @@ static void launch_rows(const uint32_t* d_sys, const uint32_t* d_snap, int lx, i
                         bool starts, cudaStream_t st)
 {
     const dim3 grid(1u << (ly - row_block_lg(ly)), d_snap ? 2 : 1);
-    row_kernel<<<grid, AN_ROW_THREADS, 0, st>>>(d_sys, d_snap, lx, ly, s->rowinfo, starts ? s->rowstart : nullptr,
-                                                walk_state(s));
+    auto kern = aligned16(d_sys) && aligned16(d_snap) ? row_kernel<false> : row_kernel<true>;
+    kern<<<grid, AN_ROW_THREADS, 0, st>>>(d_sys, d_snap, lx, ly, s->rowinfo, starts ? s->rowstart : nullptr, walk_state(s));
 }
 
 cudaError_t analysis_moments_record(const uint32_t* d_sys, const uint32_t* d_snap, int lx, int ly,
@@ -932,6 +946,7 @@ extern "C" kpzb_status kpzb_roughness_noalloc(const uint32_t* d_cbbit, int lx, i
 {
     using namespace kpzb;
     if (!d_cbbit || !out) return fail(KPZB_EINVAL, "null lattice or output");
+    if ((uintptr_t)d_cbbit & 3u) return fail(KPZB_EINVAL, "lattice not on a word boundary");
     if (lx < 8 || lx > 30 || ly < 2 || lx + ly < 14 || lx + ly > 38)
         return fail(KPZB_EINVAL, "lattice size out of range (8<=lx<=30, 14<=lx+ly<=38)");
     if (ly > NOALLOC_MAX_LY)

@@ -35,14 +35,13 @@
 namespace kpzb {
 
 // The two X-slope quadrants of a lattice (sublattice 0 at word 0, sublattice 1 at 2Q) into the
-// store's tiles: 16 bytes per tile, smax * 16 apart.
+// store's tiles: 16 bytes per tile, smax * 16 apart.  The lattice is the caller's and may start at
+// any word, so it is read word by word.
 __global__ void gram_store_kernel(const uint32_t* __restrict__ cbbit, uint64_t Q, int smax, int s, uint4* __restrict__ out)
 {
-    const uint2* a = reinterpret_cast<const uint2*>(cbbit);
-    const uint2* b = reinterpret_cast<const uint2*>(cbbit + 2 * Q);
+    const uint32_t *a = cbbit, *b = cbbit + 2 * Q;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < Q / 2; t += (uint64_t)gridDim.x * blockDim.x) {
-        const uint2 x = a[t], y = b[t];
-        out[t * (uint64_t)smax + (uint64_t)s] = make_uint4(x.x, x.y, y.x, y.y);
+        out[t * (uint64_t)smax + (uint64_t)s] = make_uint4(a[2 * t], a[2 * t + 1], b[2 * t], b[2 * t + 1]);
     }
 }
 
@@ -188,6 +187,7 @@ extern "C" kpzb_status kpzb_gram_add_device(kpzb_gram* g, const uint32_t* d_cbbi
 {
     GCHECK(g);
     if (!d_cbbit) return fail(KPZB_EINVAL, "null lattice");
+    if ((uintptr_t)d_cbbit & 3u) return fail(KPZB_EINVAL, "lattice not on a word boundary");
     if (g->n >= g->smax) return fail(KPZB_ESTATE, "snapshot capacity reached");
     const int s = g->n;
     // the snapshot's mean fixes its integer shift c_s = floor(<h>); the walk that measures it

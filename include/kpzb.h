@@ -186,7 +186,8 @@ kpzb_status kpzb_roughness_join(kpzb_handle* h, double out[8]);
  * of about 1.6 MB held by every GPU that loads the library's module.  For callers that
  * cannot allocate device memory at measurement time (their allocator owns the device, or an
  * allocation would synchronize the device inside a timing loop).  No counterpart in the
- * reference.  Limit: ly <= 16.  Calls overlapping on the GPU race on the shared scratch.
+ * reference.  Limit: ly <= 16.  d_cbbit may start at any 32-bit word of a buffer (KPZB_EINVAL
+ * off a word boundary).  Calls overlapping on the GPU race on the shared scratch.
  * Set-up: the scratch's device address is looked up once per device and CUDA context (again
  * after the caller recreates the context, e.g. by cudaDeviceReset); that first call may also
  * load the library's module with its array, so a caller whose no-allocation window must see
@@ -320,7 +321,8 @@ kpzb_status kpzb_measure_run(kpzb_handle* h, const kpzb_sampling* s, uint64_t en
 typedef struct kpzb_gram kpzb_gram;
 kpzb_status kpzb_gram_create(kpzb_gram** g, int lx, int ly, int max_snapshots, int device);
 kpzb_status kpzb_gram_destroy(kpzb_gram* g);
-/* Add a snapshot from a device ENC_CBBIT lattice (e.g. kpzb_device_ptr of an SCABit handle). */
+/* Add a snapshot from a device ENC_CBBIT lattice (e.g. kpzb_device_ptr of an SCABit handle), which
+ * may start at any 32-bit word of a buffer (KPZB_EINVAL off a word boundary). */
 kpzb_status kpzb_gram_add_device(kpzb_gram* g, const uint32_t* d_cbbit);
 kpzb_status kpzb_gram_add_host(kpzb_gram* g, const uint32_t* cbbit);
 /* G (n x n, row-major int64) of the n snapshots added so far, and the per-snapshot sums
