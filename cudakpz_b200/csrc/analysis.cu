@@ -264,7 +264,8 @@ __device__ __forceinline__ long long row_block_bases(const RowBlock* blocks, int
 //
 // The bins cover WALK_REACH heights on each side of the middle of the row starts (a surface of
 // 16384^2 has heights within about 30 of its mean at t = 10^4).  A chunk of 64 sites that leaves
-// them is summed site by site, as is a row's first chunk when the row's slopes do not close.
+// them goes by its own power sums (walk_far), as does a row's first chunk when the row's slopes
+// do not close.
 constexpr int WALK_BINS = 192;
 constexpr int WALK_REACH = WALK_BINS - 64;  // a chunk moves at most 64 from its first height
 constexpr int WALK_LUT = 256;
@@ -278,24 +279,6 @@ __device__ __forceinline__ uint32_t byte_popc(uint32_t v)
     return (v + (v >> 4)) & 0x0F0F0F0Fu;
 }
 
-struct Sums {
-    long long s1, s2, hmin, hmax;
-    double s[5];
-    __device__ void add_height(long long h)
-    {
-        s1 += h;
-        s2 += h * h;
-        const double d = (double)h, d2 = d * d, d3 = d2 * d;
-        s[0] += d3;
-        s[1] += d2 * d2;
-        s[2] += d3 * d2;
-        s[3] += d3 * d3;
-        s[4] += d3 * d3 * d;
-        hmin = min(hmin, h);
-        hmax = max(hmax, h);
-    }
-};
-
 // One word of a Partial: its value over the CTA's threads, by the warp that reads it.  Words 0, 1
 // and 4-6 are added as integers, 2 and 3 are the extremes, the rest are added in FP64.
 constexpr int PARTIAL_SUMS = 12;
@@ -305,12 +288,30 @@ __device__ __forceinline__ int partial_word(int q) { return q < 7 ? q : q + 1; }
 // memory, 12 * NT words) and a warp adds up each quantity, lane by lane and then by a tree, in the
 // same order in every call.  (Shuffling all twelve 64-bit values through every warp took 4 us.)
 template <int NT>
-__device__ __forceinline__ void cta_partial(const Partial& p, long long* buf, Partial* out)
+__device__ __forceinline__ void put_partial(const Partial& p, long long* buf)
 {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const long long* pw = reinterpret_cast<const long long*>(&p);
 #pragma unroll
     for (int q = 0; q < PARTIAL_SUMS; ++q) buf[q * NT + threadIdx.x] = pw[partial_word(q)];
+}
+
+// The same values added to what this thread has stored.
+template <int NT>
+__device__ __forceinline__ void add_partial(const Partial& p, long long* buf)
+{
+    const long long* pw = reinterpret_cast<const long long*>(&p);
+#pragma unroll
+    for (int q = 0; q < PARTIAL_SUMS; ++q) {
+        long long& v = buf[q * NT + threadIdx.x];
+        const long long x = pw[partial_word(q)];
+        v = q == 2 ? min(v, x) : q == 3 ? max(v, x) : q < 7 ? v + x : __double_as_longlong(__longlong_as_double(v) + __longlong_as_double(x));
+    }
+}
+
+template <int NT>
+__device__ __forceinline__ void cta_reduce(const long long* buf, Partial* out)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     __syncthreads();
     if (wid < PARTIAL_SUMS) {
         const long long* v = buf + wid * NT + lane;
@@ -340,77 +341,63 @@ __device__ __forceinline__ Partial empty_partial()
     return p;
 }
 
-// CORR: also the correlator's sums against `snap` (cross sum of heights, agreeing slopes).  Its
-// heights relative to the two lattices' middles are built as biased bytes from a table of
-// the patterns' cumulative steps and multiplied four sites at a time (dp4a).
-constexpr int walk_threads(bool corr) { return corr ? 768 : 1024; }  // 85 and 64 registers
+// What a warp of the walk needs to find the chunks of its items: rows of parity `par`, or quarters of
+// them where rows are long.
+struct WalkGeom {
+    const uint32_t *sys, *snap;
+    const int4* rowinfo;      // of the system; the snapshot's 2^ly further on
+    const int64_t* rowstart;
+    const long long *base, *base_s;  // heights at the start of every row block
+    const uint32_t* step4;           // table of add_chunk
+    long long mid, mid_s;            // middles of the row starts
+    int lx, ly, par;
+    uint64_t item, step;  // the warp's first item and the distance to its next
+};
 
-template <bool CORR>
-__global__ void __launch_bounds__(walk_threads(CORR), 1)
-walk_kernel(const uint32_t* __restrict__ sys, const uint32_t* __restrict__ snap, int lx, int ly,
-            const int4* __restrict__ rowinfo, const int64_t* __restrict__ rowstart, Partial* __restrict__ partials,
-            Partial* __restrict__ out, WalkState* ws)
+// Items of one row parity.
+__host__ __device__ inline uint64_t walk_items(int lx, int ly)
 {
-    constexpr int NT = walk_threads(CORR), NWARP = NT / 32;
-    extern __shared__ __align__(16) uint32_t hist[];  // [height bin][pattern ^ bin]
-    __shared__ uint2 lut[CORR ? WALK_LUT : 1];
-    __shared__ long long base_s[CORR ? 2 : 1][AN_MAX_BLOCKS];
-    __shared__ int used[2];  // first and last bin of a chunk's first group
-    __shared__ bool last;
+    const uint64_t Wr = 1ull << (lx - 6), rows = 1ull << ly;
+    return Wr >= AN_PART_WORDS ? 2 * rows : rows / 2 / (Wr < 32 ? 32 / Wr : 1);
+}
 
-    const uint64_t Wr = 1ull << (lx - 6);
-    const uint64_t Q = 1ull << (lx + ly - 6);
-    const uint64_t rows = 1ull << ly;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int par = (int)(blockIdx.x & 1);            // row parity of this CTA
-    const uint64_t nctas = gridDim.x >> 1, cta = blockIdx.x >> 1;
-    const int64_t* rowstart_s = rowstart + rows;
-    const int4* rowinfo_s = rowinfo + rows;
-
-    if (threadIdx.x == 0) {
-        used[0] = WALK_BINS;
-        used[1] = -1;
+// One chunk of 64 sites: its X-slope words (even-x and odd-x), the height before it relative to
+// the middle of the row starts, and the same of the snapshot; first: it starts at x = 0.
+struct Chunk {
+    uint32_t e, o, es, os;
+    long long rel, rel_s;
+    int sum_r, sum_s;  // slope sums of the chunk's row
+    bool first;
+    __device__ bool binned() const { return rel >= -WALK_REACH && rel < WALK_REACH && !(first && sum_r != 0); }
+    // u and v as bytes: no carry while the chunk stays within [-127, 127] of the middles
+    __device__ bool bytes() const
+    {
+        return rel >= -63 && rel <= 63 && rel_s >= -63 && rel_s <= 63 && !(first && (sum_r | sum_s) != 0);
     }
-    for (int i = threadIdx.x; i < WALK_BINS * 64; i += NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (CORR && threadIdx.x < WALK_LUT) {
-        // byte j: 8 + sum_{k <= j} (2 bit_k - 1), the pattern's even-x bits low, odd-x bits high
-        int cum = 8;
-        uint32_t w[2] = {0u, 0u};
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            cum += 2 * (int)((threadIdx.x >> ((j & 1 ? 4 : 0) + (j >> 1))) & 1u) - 1;
-            w[j >> 2] |= (uint32_t)cum << (8 * (j & 3));
-        }
-        lut[threadIdx.x] = make_uint2(w[0], w[1]);
-    }
-    const int lgb = row_block_lg(ly), nblk = (int)(rows >> lgb);
-    const long long mid = row_block_bases<NT>(ws->block[0], nblk, base_s[0]);
-    const long long mid_s = CORR ? row_block_bases<NT>(ws->block[1], nblk, base_s[CORR ? 1 : 0]) : 0;
-    // bin s holds groups with height H0 + 2 s before their first site; H0 has the parity of the
-    // heights before x = 0 of this CTA's rows, Hs(y) - e0
-    const long long first_h = rowstart[par] - 1;  // block 0 starts at 0; e0 = +-1: either way the same parity
-    const long long H0 = mid - WALK_BINS + ((mid - WALK_BINS - first_h) & 1);
-    __syncthreads();
+};
 
-    Sums slow{0, 0, 0x7fffffffffffffffll, -0x7fffffffffffffffll, {0, 0, 0, 0, 0}};
-    int bin_lo = WALK_BINS, bin_hi = -1;
-    // correlator: sums over sites of u v and of v, u = h - mid + 128 and v = h' - mid' + 128
-    long long uv_sum = 0, v_sum = 0, agree = 0;
-
+// Hands every chunk of the warp's items to `chunk`, with the number of agreeing Y slopes.
+template <bool CORR, class F>
+__device__ __forceinline__ void walk_chunks(const WalkGeom& g, F&& chunk)
+{
+    const uint64_t Wr = 1ull << (g.lx - 6);
+    const uint64_t Q = 1ull << (g.lx + g.ly - 6);
+    const uint64_t rows = 1ull << g.ly;
+    const int lane = threadIdx.x & 31, lgb = row_block_lg(g.ly);
     const int wl = (int)(Wr < 32 ? Wr : 32);      // lanes per row
     const int rpw = 32 / wl;                      // rows per warp
     const int parts = Wr >= AN_PART_WORDS ? 4 : 1;
     const uint64_t pw = Wr / parts;               // words per part
-    const uint64_t items = rows / 2 / rpw * parts;
+    const uint64_t items = walk_items(g.lx, g.ly);
     const int sub = lane % wl;
-    const uint64_t be = par ? 2 * Q : 0, bo = par ? 0 : 2 * Q;
+    const uint64_t be = g.par ? 2 * Q : 0, bo = g.par ? 0 : 2 * Q;
 
-    for (uint64_t it = cta * NWARP + wid; it < items; it += nctas * NWARP) {
+    for (uint64_t it = g.item; it < items; it += g.step) {
         const int part = (int)(it % parts);
-        const uint64_t y = 2 * (it / parts * rpw + lane / wl) + par;
+        const uint64_t y = 2 * (it / parts * rpw + lane / wl) + g.par;
         const uint64_t off = y * Wr + part * pw;
-        const uint32_t *pe = sys + be + off, *po = sys + bo + off;
-        const uint32_t *qe = snap + be + off, *qo = snap + bo + off;
+        const uint32_t *pe = g.sys + be + off, *po = g.sys + bo + off;
+        const uint32_t *qe = g.snap + be + off, *qo = g.snap + bo + off;
         // the next chunk's words: X of both sublattices, for the correlator Y and the snapshot's
         uint32_t w[CORR ? 8 : 2];
         auto load = [&](uint64_t c) {
@@ -429,32 +416,33 @@ walk_kernel(const uint32_t* __restrict__ sys, const uint32_t* __restrict__ snap,
         // height before the part's first site: Hs - e0 + 2 (bits set before it) - sites
         auto before = [&](const int4& r) { return part == 0 ? 0 : part == 1 ? r.x : part == 2 ? r.y : r.z; };
         const long long back = (long long)(64 * pw * part);
-        const int4 ri = rowinfo[y];
-        const long long Hs = rowstart[y] + base_s[0][y >> lgb];
-        long long H = Hs - (2 * (int)(sys[be + y * Wr] & 1u) - 1) + 2 * (long long)before(ri) - back;
+        const int4 ri = g.rowinfo[y];
+        long long H = g.rowstart[y] + g.base[y >> lgb] - (2 * (int)(g.sys[be + y * Wr] & 1u) - 1) +
+                      2 * (long long)before(ri) - back - g.mid;
         long long Hsn = 0;
-        int sum_s = 0;
+        Chunk ch{};
+        ch.sum_r = row_sum(ri.w);
         if (CORR) {
-            const int4 si = rowinfo_s[y];
-            sum_s = row_sum(si.w);
-            Hsn = rowstart_s[y] + base_s[CORR ? 1 : 0][y >> lgb] - (2 * (int)(snap[be + y * Wr] & 1u) - 1) +
-                  2 * (long long)before(si) - back;
+            const int4 si = g.rowinfo[rows + y];
+            ch.sum_s = row_sum(si.w);
+            Hsn = g.rowstart[rows + y] + g.base_s[y >> lgb] - (2 * (int)(g.snap[be + y * Wr] & 1u) - 1) +
+                  2 * (long long)before(si) - back - g.mid_s;
         }
-        const int sum_r = row_sum(ri.w);
         for (uint64_t c = sub; c < pw; c += wl) {
-            const uint32_t e = w[0], o = w[1];
-            uint32_t es = 0, os = 0;
+            ch.e = w[0];
+            ch.o = w[1];
+            int eq = 0;
             if (CORR) {
-                es = w[2];
-                os = w[3];
-                agree += 2 * (__popc(~(e ^ es)) + __popc(~(o ^ os)) + __popc(~(w[4] ^ w[6])) + __popc(~(w[5] ^ w[7]))) - 128;
+                ch.es = w[2];
+                ch.os = w[3];
+                eq = __popc(~(w[4] ^ w[6])) + __popc(~(w[5] ^ w[7]));
             }
             if (c + wl < pw) load(c + wl);
             // the chunk's total step and the heights before it, in the row's lanes
-            const int n = __popc(e) + __popc(o) - 32;
+            const int n = __popc(ch.e) + __popc(ch.o) - 32;
             int incl = n;
             int ns = 0, incl_s = 0;
-            if (CORR) incl_s = ns = __popc(es) + __popc(os) - 32;
+            if (CORR) incl_s = ns = __popc(ch.es) + __popc(ch.os) - 32;
             for (int k = 1; k < wl; k <<= 1) {
                 const int a = __shfl_up_sync(0xffffffffu, incl, k, wl);
                 if (sub >= k) incl += a;
@@ -463,83 +451,260 @@ walk_kernel(const uint32_t* __restrict__ sys, const uint32_t* __restrict__ snap,
                     if (sub >= k) incl_s += b;
                 }
             }
-            const long long h0 = H + 2 * (incl - n);
+            ch.first = part == 0 && c == 0;
+            ch.rel = H + 2 * (incl - n);
             H += 2 * __shfl_sync(0xffffffffu, incl, wl - 1, wl);
-            // patterns of the even and the odd groups, a byte each, and their set bits
-            const uint32_t A = (e & 0x0F0F0F0Fu) | ((o & 0x0F0F0F0Fu) << 4);
-            const uint32_t B = ((e >> 4) & 0x0F0F0F0Fu) | (o & 0xF0F0F0F0u);
-            const uint32_t pa = byte_popc(A), pb = byte_popc(B);
-            const bool open_row = part == 0 && c == 0 && sum_r != 0;
-            const long long rel = h0 - mid;
-            if (rel >= -WALK_REACH && rel < WALK_REACH && !open_row) {
-                // absolute bin of each group: s0 + bits before it - 4 per group before it
-                const int s0 = (int)(h0 - H0) >> 1;
-                bin_lo = min(bin_lo, s0);
-                bin_hi = max(bin_hi, s0);
-                const uint32_t sa = (pa + pb) * 0x01010100u + (uint32_t)s0 * 0x01010101u - 0x18100800u;
-                const uint32_t sb = sa + pa - 0x04040404u;
-                // the pattern is XORed with the bin so that equal patterns at different heights
-                // lie in different banks
-                const uint32_t xa = A ^ sa, xb = B ^ sb;
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const uint32_t ta = __byte_perm(xa, sa, i ? 0x7362 : 0x5140);
-                    const uint32_t tb = __byte_perm(xb, sb, i ? 0x7362 : 0x5140);
-                    atomicAdd(&hist[ta & 0xFFFFu], 1u);
-                    atomicAdd(&hist[tb & 0xFFFFu], 1u);
-                    atomicAdd(&hist[ta >> 16], 1u);
-                    atomicAdd(&hist[tb >> 16], 1u);
-                }
-            } else {
-                long long h = h0;
-#pragma unroll 1
-                for (int i = 0; i < 64; ++i) {
-                    h += 2 * (long long)((((i & 1) ? o : e) >> (i >> 1)) & 1u) - 1;
-                    slow.add_height(i == 0 && open_row ? Hs + sum_r : h);
-                }
-            }
             if (CORR) {
-                const long long hs0 = Hsn + 2 * (incl_s - ns);
+                ch.rel_s = Hsn + 2 * (incl_s - ns);
                 Hsn += 2 * __shfl_sync(0xffffffffu, incl_s, wl - 1, wl);
-                const long long rel_s = hs0 - mid_s;
-                const bool open_s = part == 0 && c == 0 && sum_s != 0;
-                // u and v as bytes: no carry while the chunk stays within [-127, 127] of the middles
-                if (rel >= -63 && rel <= 63 && rel_s >= -63 && rel_s <= 63 && !open_row && !open_s) {
-                    const uint32_t As = (es & 0x0F0F0F0Fu) | ((os & 0x0F0F0F0Fu) << 4);
-                    const uint32_t Bs = ((es >> 4) & 0x0F0F0F0Fu) | (os & 0xF0F0F0F0u);
-                    uint32_t b = (uint32_t)((int)rel + 120) * 0x01010101u, bs = (uint32_t)((int)rel_s + 120) * 0x01010101u;
-                    unsigned int uv = 0, vv = 0;
-#pragma unroll
-                    for (int g = 0; g < 8; ++g) {
-                        const uint2 T = lut[((g & 1 ? B : A) >> (8 * (g >> 1))) & 0xFFu];
-                        const uint2 Ts = lut[((g & 1 ? Bs : As) >> (8 * (g >> 1))) & 0xFFu];
-                        const uint32_t u0 = b + T.x, u1 = b + T.y, v0 = bs + Ts.x, v1 = bs + Ts.y;
-                        uv = __dp4a(u0, v0, uv);
-                        uv = __dp4a(u1, v1, uv);
-                        vv = __dp4a(v0, 0x01010101u, vv);
-                        vv = __dp4a(v1, 0x01010101u, vv);
-                        // the next group starts at this one's last height: byte 3, less the 8 of the bias
-                        b = __byte_perm(u1, 0u, 0x3333) - 0x08080808u;
-                        bs = __byte_perm(v1, 0u, 0x3333) - 0x08080808u;
-                    }
-                    uv_sum += uv;
-                    v_sum += vv;
-                } else {
-                    long long r = rel + 128, s = rel_s + 128;
-#pragma unroll 1
-                    for (int i = 0; i < 64; ++i) {
-                        r += 2 * (long long)((((i & 1) ? o : e) >> (i >> 1)) & 1u) - 1;
-                        s += 2 * (long long)((((i & 1) ? os : es) >> (i >> 1)) & 1u) - 1;
-                        // x = 0 takes the height its row ends with
-                        const long long a = i == 0 && part == 0 && c == 0 ? r + sum_r : r;
-                        const long long b = i == 0 && part == 0 && c == 0 ? s + sum_s : s;
-                        uv_sum += a * b;
-                        v_sum += b;
-                    }
-                }
             }
+            chunk(ch, eq);
         }
     }
+}
+
+// A chunk of 64 sites outside the bins: its heights are b + d_i with b the height before its first
+// site and |d_i| <= 64, so the power sums of d are whole numbers below 2^49, exact in FP64, and the
+// sums of h^k follow once per chunk by the binomial expansion.  The d_i come four at a time as biased
+// bytes from a table of the four-site patterns (even-x bits in bits 0-1, odd-x bits in bits 2-3).
+// Nine FP64 and about six integer operations a site on two pipes, where powers in 32- and 64-bit
+// integers kept one pipe busy for about 40 cycles a warp.  open: the chunk's first site is x = 0 of a
+// row whose slopes sum to `row`, not 0; its height is b + d_0 + row, the one its row ends with, and it
+// is left out of the power sums.
+__device__ __forceinline__ void add_chunk(Partial& s, uint32_t e, uint32_t o, long long b, bool open, int row,
+                                          const uint32_t* step4)
+{
+    const uint32_t A = (e & 0x33333333u) | ((o & 0x33333333u) << 2), B = ((e >> 2) & 0x33333333u) | (o & 0xCCCCCCCCu);
+    int a1 = 0, a2 = 0, dmin = 255, dmax = 0;
+    double A3 = 0, A4 = 0, A5 = 0, A6 = 0, A7 = 0;
+    uint32_t base = 0x7C7C7C7Cu;  // bytes: d before the four sites, + 128 - 4 (the table's bias)
+#pragma unroll 4
+    for (int g = 0; g < 16; ++g) {
+        const uint32_t u = base + step4[((g & 1 ? B : A) >> (4 * (g >> 1))) & 15u];
+        base = __byte_perm(u, 0u, 0x3333) - 0x04040404u;
+        const int x = (int)(u ^ 0x80808080u);  // the four d as signed bytes
+        a1 = __dp4a(x, 0x01010101, a1);
+        a2 = __dp4a(x, x, a2);
+        int v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            v[j] = (int)__byte_perm(u, 0u, 0x4440 | j);  // d + 128
+            const double d = __hiloint2double(0x43300000, v[j]) - 4503599627370624.0;  // 2^52 + 128
+            const double d2 = d * d, d4 = d2 * d2, d5 = d4 * d;
+            A3 += d2 * d;
+            A4 += d4;
+            A5 += d5;
+            A6 += d4 * d2;
+            A7 += d5 * d2;
+        }
+        const int v0 = g == 0 && open ? v[1] : v[0];
+        dmin = __vimin3_s32(__vimin3_s32(dmin, v0, v[1]), v[2], v[3]);
+        dmax = __vimax3_s32(__vimax3_s32(dmax, v0, v[1]), v[2], v[3]);
+    }
+    dmin -= 128;
+    dmax -= 128;
+    const int first = 2 * (int)(e & 1u) - 1;  // d_0
+    if (open) {
+        a1 -= first;
+        a2 -= 1;
+        A3 -= first;
+        A4 -= 1;
+        A5 -= first;
+        A6 -= 1;
+        A7 -= first;
+    }
+    const int n = open ? 63 : 64;
+    s.s1 += (long long)n * b + a1;
+    s.s2 += (long long)n * b * b + 2 * b * a1 + a2;
+    s.hmin = min(s.hmin, b + dmin);
+    s.hmax = max(s.hmax, b + dmax);
+    const double B1 = (double)b, B2 = B1 * B1, B3 = B2 * B1, B4 = B2 * B2, B5 = B4 * B1, B6 = B3 * B3, B7 = B6 * B1;
+    const double N = n, A1 = a1, A2 = a2;
+    s.s[0] += N * B3 + 3.0 * B2 * A1 + 3.0 * B1 * A2 + A3;
+    s.s[1] += N * B4 + 4.0 * B3 * A1 + 6.0 * B2 * A2 + 4.0 * B1 * A3 + A4;
+    s.s[2] += N * B5 + 5.0 * B4 * A1 + 10.0 * B3 * A2 + 10.0 * B2 * A3 + 5.0 * B1 * A4 + A5;
+    s.s[3] += N * B6 + 6.0 * B5 * A1 + 15.0 * B4 * A2 + 20.0 * B3 * A3 + 15.0 * B2 * A4 + 6.0 * B1 * A5 + A6;
+    s.s[4] += N * B7 + 7.0 * B6 * A1 + 21.0 * B5 * A2 + 35.0 * B4 * A3 + 35.0 * B3 * A4 + 21.0 * B2 * A5 + 7.0 * B1 * A6 + A7;
+    if (open) {
+        const long long hf = b + first + row;
+        const double h = (double)hf, h2 = h * h, h3 = h2 * h;
+        s.s1 += hf;
+        s.s2 += hf * hf;
+        s.s[0] += h3;
+        s.s[1] += h2 * h2;
+        s.s[2] += h3 * h2;
+        s.s[3] += h3 * h3;
+        s.s[4] += h3 * h3 * h;
+        s.hmin = min(s.hmin, hf);
+        s.hmax = max(s.hmax, hf);
+    }
+}
+
+// Sums over a chunk of u v (x) and of v (y), u = 128 + rel + d_i and v = 128 + rel_s + d'_i from the steps
+// of the two lattices' slope words; x = 0 takes the height its row ends with, the row's sum further.
+__device__ __forceinline__ void add_cross(longlong2& sum, const Chunk& c)
+{
+    int d = 0, ds = 0, sd = 0, sds = 0, sdd = 0;
+    auto add = [&](uint32_t b, uint32_t bs) {
+        d += 2 * (int)(b & 1u) - 1;
+        ds += 2 * (int)(bs & 1u) - 1;
+        sd += d;
+        sds += ds;
+        sdd += d * ds;
+    };
+#pragma unroll 4
+    for (int i = 0; i < 32; ++i) {
+        add(c.e >> i, c.es >> i);
+        add(c.o >> i, c.os >> i);
+    }
+    const long long r = 128 + c.rel, q = 128 + c.rel_s;
+    sum.x += 64 * r * q + r * sds + q * sd + sdd;
+    sum.y += 64 * q + sds;
+    if (c.first) {
+        const long long u = r + 2 * (int)(c.e & 1u) - 1, v = q + 2 * (int)(c.es & 1u) - 1;
+        sum.x += (u + c.sum_r) * (v + c.sum_s) - u * v;
+        sum.y += c.sum_s;
+    }
+}
+
+// The chunks that the walk over the bins leaves out, in a second walk by the warps that met one: as
+// code of that walk they cost a tenth of its time in registers, although surfaces in their growth
+// regime have none.  A pyramid of 16384^2, nearly all of it outside the bins: roughness 310 us, a
+// correlation of random words 470 us (490 and 950 with the powers of every height in the first walk;
+// 330 and 690 by chunks alone, without bins).  cross: the correlator's sums of u v and v over the
+// chunks without bytes.
+template <bool CORR>
+__device__ __noinline__ void walk_far(const WalkGeom& g, Partial* sums, longlong2* cross)
+{
+    walk_chunks<CORR>(g, [&](const Chunk& c, int) {
+        if (!c.binned()) add_chunk(*sums, c.e, c.o, c.rel + g.mid, c.first && c.sum_r != 0, c.sum_r, g.step4);
+        if (CORR && !c.bytes()) add_cross(*cross, c);
+    });
+}
+
+// CORR: also the correlator's sums against `snap` (cross sum of heights, agreeing slopes).  Its
+// heights relative to the two lattices' middles are built as biased bytes from a table of
+// the patterns' cumulative steps and multiplied four sites at a time (dp4a).
+constexpr int walk_threads(bool corr) { return corr ? 768 : 1024; }  // 85 and 64 registers
+
+template <bool CORR>
+__global__ void __launch_bounds__(walk_threads(CORR), 1)
+walk_kernel(const uint32_t* __restrict__ sys, const uint32_t* __restrict__ snap, int lx, int ly,
+            const int4* __restrict__ rowinfo, const int64_t* __restrict__ rowstart, Partial* __restrict__ partials,
+            Partial* __restrict__ out, WalkState* ws)
+{
+    constexpr int NT = walk_threads(CORR), NWARP = NT / 32;
+    extern __shared__ __align__(16) uint32_t hist[];  // [height bin][pattern ^ bin]
+    __shared__ uint2 lut[CORR ? WALK_LUT : 1];
+    __shared__ long long base_s[CORR ? 2 : 1][AN_MAX_BLOCKS];
+    __shared__ uint32_t step4[16];
+    __shared__ int used[2];  // first and last bin of a chunk's first group
+    __shared__ bool last;
+
+    const uint64_t rows = 1ull << ly;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int par = (int)(blockIdx.x & 1);            // row parity of this CTA
+    const uint64_t nctas = gridDim.x >> 1, cta = blockIdx.x >> 1;
+
+    if (threadIdx.x == 0) {
+        used[0] = WALK_BINS;
+        used[1] = -1;
+    }
+    for (int i = threadIdx.x; i < WALK_BINS * 64; i += NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (CORR && threadIdx.x < WALK_LUT) {
+        // byte j: 8 + sum_{k <= j} (2 bit_k - 1), the pattern's even-x bits low, odd-x bits high
+        int cum = 8;
+        uint32_t w[2] = {0u, 0u};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            cum += 2 * (int)((threadIdx.x >> ((j & 1 ? 4 : 0) + (j >> 1))) & 1u) - 1;
+            w[j >> 2] |= (uint32_t)cum << (8 * (j & 3));
+        }
+        lut[threadIdx.x] = make_uint2(w[0], w[1]);
+    }
+    if (threadIdx.x < 16) {
+        // byte j: 4 + sum_{k <= j} (2 bit_k - 1)
+        int cum = 4;
+        uint32_t w = 0;
+        for (int j = 0; j < 4; ++j) {
+            cum += 2 * (int)((threadIdx.x >> ((j & 1 ? 2 : 0) + (j >> 1))) & 1u) - 1;
+            w |= (uint32_t)cum << (8 * j);
+        }
+        step4[threadIdx.x] = w;
+    }
+    const int lgb = row_block_lg(ly), nblk = (int)(rows >> lgb);
+    const long long mid = row_block_bases<NT>(ws->block[0], nblk, base_s[0]);
+    const long long mid_s = CORR ? row_block_bases<NT>(ws->block[1], nblk, base_s[CORR ? 1 : 0]) : 0;
+    // bin s holds groups with height H0 + 2 s before their first site; H0 has the parity of the
+    // heights before x = 0 of this CTA's rows, Hs(y) - e0
+    const long long first_h = rowstart[par] - 1;  // block 0 starts at 0; e0 = +-1: either way the same parity
+    const long long H0 = mid - WALK_BINS + ((mid - WALK_BINS - first_h) & 1);
+    const int h0_rel = (int)(mid - H0);
+    __syncthreads();
+
+    int bin_lo = WALK_BINS, bin_hi = -1;
+    bool far = false;  // this lane has met a chunk that the bins (or the correlator's bytes) do not reach
+    // correlator: sums over sites of u v and of v, u = h - mid + 128 and v = h' - mid' + 128
+    long long uv_sum = 0, v_sum = 0, agree = 0;
+
+    // items are dealt to the CTAs in turn, so that few of them still use every SM (2^20 x 2^8 sites:
+    // roughness 210 -> 135 us)
+    const WalkGeom geom{sys, snap, rowinfo, rowstart, base_s[0], base_s[CORR ? 1 : 0], step4, mid, mid_s, lx, ly, par,
+                        (uint64_t)wid * nctas + cta, nctas * NWARP};
+    walk_chunks<CORR>(geom, [&](const Chunk& c, int eq) {
+        // patterns of the even and the odd groups, a byte each, and their set bits
+        const uint32_t A = (c.e & 0x0F0F0F0Fu) | ((c.o & 0x0F0F0F0Fu) << 4);
+        const uint32_t B = ((c.e >> 4) & 0x0F0F0F0Fu) | (c.o & 0xF0F0F0F0u);
+        const uint32_t pa = byte_popc(A), pb = byte_popc(B);
+        if (c.binned()) {
+            // absolute bin of each group: s0 + bits before it - 4 per group before it
+            const int s0 = ((int)c.rel + h0_rel) >> 1;
+            bin_lo = min(bin_lo, s0);
+            bin_hi = max(bin_hi, s0);
+            const uint32_t sa = (pa + pb) * 0x01010100u + (uint32_t)s0 * 0x01010101u - 0x18100800u;
+            const uint32_t sb = sa + pa - 0x04040404u;
+            // the pattern is XORed with the bin so that equal patterns at different heights
+            // lie in different banks
+            const uint32_t xa = A ^ sa, xb = B ^ sb;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const uint32_t ta = __byte_perm(xa, sa, i ? 0x7362 : 0x5140);
+                const uint32_t tb = __byte_perm(xb, sb, i ? 0x7362 : 0x5140);
+                atomicAdd(&hist[ta & 0xFFFFu], 1u);
+                atomicAdd(&hist[tb & 0xFFFFu], 1u);
+                atomicAdd(&hist[ta >> 16], 1u);
+                atomicAdd(&hist[tb >> 16], 1u);
+            }
+        } else {
+            far = true;
+        }
+        if (CORR) {
+            agree += 2 * (eq + __popc(~(c.e ^ c.es)) + __popc(~(c.o ^ c.os))) - 128;
+            if (c.bytes()) {
+                const uint32_t As = (c.es & 0x0F0F0F0Fu) | ((c.os & 0x0F0F0F0Fu) << 4);
+                const uint32_t Bs = ((c.es >> 4) & 0x0F0F0F0Fu) | (c.os & 0xF0F0F0F0u);
+                uint32_t b = (uint32_t)((int)c.rel + 120) * 0x01010101u, bs = (uint32_t)((int)c.rel_s + 120) * 0x01010101u;
+                unsigned int uv = 0, vv = 0;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    const uint2 T = lut[((g & 1 ? B : A) >> (8 * (g >> 1))) & 0xFFu];
+                    const uint2 Ts = lut[((g & 1 ? Bs : As) >> (8 * (g >> 1))) & 0xFFu];
+                    const uint32_t u0 = b + T.x, u1 = b + T.y, v0 = bs + Ts.x, v1 = bs + Ts.y;
+                    uv = __dp4a(u0, v0, uv);
+                    uv = __dp4a(u1, v1, uv);
+                    vv = __dp4a(v0, 0x01010101u, vv);
+                    vv = __dp4a(v1, 0x01010101u, vv);
+                    // the next group starts at this one's last height: byte 3, less the 8 of the bias
+                    b = __byte_perm(u1, 0u, 0x3333) - 0x08080808u;
+                    bs = __byte_perm(v1, 0u, 0x3333) - 0x08080808u;
+                }
+                uv_sum += uv;
+                v_sum += vv;
+            } else {
+                far = true;
+            }
+        }
+    });
     bin_lo = __reduce_min_sync(0xffffffffu, bin_lo);
     bin_hi = __reduce_max_sync(0xffffffffu, bin_hi);
     if (lane == 0) {
@@ -604,21 +769,28 @@ walk_kernel(const uint32_t* __restrict__ sys, const uint32_t* __restrict__ snap,
             }
         }
     }
-    acc.s1 += slow.s1;
-    acc.s2 += slow.s2;
-    acc.hmin = min(acc.hmin, slow.hmin);
-    acc.hmax = max(acc.hmax, slow.hmax);
-    for (int k = 0; k < 5; ++k) acc.s[k] += slow.s[k];
+    // summed over all sites, sum h h' = sum u v + (mid - 128) sum v + (mid' - 128) sum h; the last term
+    // is linear in s1, so every thread adds its share of it
+    auto correlate = [&](Partial& p, long long uv, long long v) {
+        p.cross = uv + (mid - 128) * v + (mid_s - 128) * p.s1;
+        p.snap_s1 = v;  // less (128 - mid') per site, below
+    };
     if (CORR) {
-        // summed over all sites, sum h h' = sum u v + (mid - 128) sum v + (mid' - 128) sum h; the
-        // last term is linear in s1, so every thread adds its share of it
-        acc.cross = uv_sum + (mid - 128) * v_sum + (mid_s - 128) * acc.s1;
+        correlate(acc, uv_sum, v_sum);
         acc.agree = agree;
-        acc.snap_s1 = v_sum;  // less (128 - mid') per site, below
     }
     __syncthreads();  // the counts have been read: their memory takes the values to add up
     long long* buf = reinterpret_cast<long long*>(hist);
-    cta_partial<NT>(acc, buf, &partials[blockIdx.x]);
+    put_partial<NT>(acc, buf);
+    if (__any_sync(0xffffffffu, far)) {
+        Partial rest = empty_partial();
+        longlong2 cross = make_longlong2(0, 0);
+        const WalkGeom again = geom;
+        walk_far<CORR>(again, &rest, &cross);
+        if (CORR) correlate(rest, cross.x, cross.y);
+        add_partial<NT>(rest, buf);
+    }
+    cta_reduce<NT>(buf, &partials[blockIdx.x]);
     if (threadIdx.x == 0) {
         __threadfence();  // the CTA's partial, ordered before this by the barrier
         last = atomicAdd(&ws->ticket, 1u) == gridDim.x - 1;
@@ -634,7 +806,8 @@ walk_kernel(const uint32_t* __restrict__ sys, const uint32_t* __restrict__ snap,
 #pragma unroll
         for (int k = 0; k < (int)(sizeof(Partial) / 16); ++k) d[k] = __ldcg(q + k);
     }
-    cta_partial<NT>(acc, buf, out);
+    put_partial<NT>(acc, buf);
+    cta_reduce<NT>(buf, out);
     if (CORR && threadIdx.x == 0) out->snap_s1 += (mid_s - 128) * (long long)(rows << lx);
 }
 
@@ -708,12 +881,10 @@ cudaError_t analysis_moments_record(const uint32_t* d_sys, const uint32_t* d_sna
                                     AnalysisScratch* s, void* d_rec, cudaStream_t st)
 {
     launch_rows(d_sys, d_snap, lx, ly, s, true, st);
-    // CTAs per row parity, at most half the SMs
-    const uint64_t Wr = 1ull << (lx - 6);
-    const uint64_t items = Wr >= AN_PART_WORDS ? (1ull << ly) * 2 : (1ull << ly) / 2 / (Wr < 32 ? 32 / Wr : 1);
+    // CTAs per row parity: one item each as long as that is at most half the SMs
+    const uint64_t items = walk_items(lx, ly);
     const unsigned threads = walk_threads(d_snap != nullptr);
-    const uint64_t want = (items + threads / 32 - 1) / (threads / 32);
-    const unsigned grid = 2 * (unsigned)(want < AN_MAX_GRID / 2 ? want : AN_MAX_GRID / 2);
+    const unsigned grid = 2 * (unsigned)(items < AN_MAX_GRID / 2 ? items : AN_MAX_GRID / 2);
     auto kern = d_snap ? walk_kernel<true> : walk_kernel<false>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_SMEM);
     if (e != cudaSuccess) return e;
