@@ -881,10 +881,12 @@ cudaError_t analysis_moments_record(const uint32_t* d_sys, const uint32_t* d_sna
                                     AnalysisScratch* s, void* d_rec, cudaStream_t st)
 {
     launch_rows(d_sys, d_snap, lx, ly, s, true, st);
-    // CTAs per row parity: one item each as long as that is at most half the SMs
+    // CTAs per row parity: a warp for each of their four schedulers as long as that is at most half
+    // the SMs
     const uint64_t items = walk_items(lx, ly);
     const unsigned threads = walk_threads(d_snap != nullptr);
-    const unsigned grid = 2 * (unsigned)(items < AN_MAX_GRID / 2 ? items : AN_MAX_GRID / 2);
+    const uint64_t want = (items + 3) / 4;
+    const unsigned grid = 2 * (unsigned)(want < AN_MAX_GRID / 2 ? want : AN_MAX_GRID / 2);
     auto kern = d_snap ? walk_kernel<true> : walk_kernel<false>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_SMEM);
     if (e != cudaSuccess) return e;
