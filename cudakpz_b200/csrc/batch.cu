@@ -57,7 +57,10 @@ struct PassState {
     uint32_t err;     // set when a bounded wait expired
 };
 
-template <int THREADS>
+// MODE: DEC_ANY, or DEC_ANY_FEW for batches whose rates need at most four random planes: the code
+// of the general decision costs the others a tenth of their time in registers (8 replicas of 2048^2
+// at (0.75,0.25): 19.2 against 17.4 us a MCS).
+template <int THREADS, int MODE>
 __global__ void __launch_bounds__(THREADS)
 batch_pass_kernel(const RepDesc* __restrict__ reps, const Item* __restrict__ items, int nitems,
                   PassState* st, int k)
@@ -88,7 +91,7 @@ batch_pass_kernel(const RepDesc* __restrict__ reps, const Item* __restrict__ ite
                          r.resident != 0, t0, r.key, r.stream, r.tp, r.tq};
         // rates differ between replicas of one launch: the run-time decision mode (a per-item
         // dispatch to rate-specialised copies measured 2-5 % slower: larger code, more registers)
-        if (!scabit_band<-1, true, false, THREADS>(smem, ctl, g, nd, nr, &st->err)) return;
+        if (!scabit_band<MODE, true, false, THREADS>(smem, ctl, g, nd, nr, &st->err)) return;
         phase ^= 1u;
     }
 }
@@ -120,6 +123,7 @@ struct kpzb_batch {
     int k = 8;                   // MCS per pass
     int chunk = 8;               // passes per graph replay
     int cps = 1;                 // CTAs per SM (1: 512 threads, 2 or 3: 256 threads each)
+    bool general = false;        // some replica's rates need more than four random planes
     bool planned = false;        // k and cps set by the caller or the tuner (else tuned on first MCS)
     cudaGraphExec_t graph = nullptr;
     AnalysisScratch an{};
@@ -188,12 +192,10 @@ static kpzb_status batch_layout(kpzb_batch* b)
 
 static cudaError_t enqueue_pass(kpzb_batch* b)
 {
-    if (b->cps <= 1)
-        batch_pass_kernel<BATCH_THREADS><<<b->sm_count, BATCH_THREADS, BATCH_SMEM, b->st>>>(
-            b->d_reps, b->d_items, b->nitems, b->d_state, b->k);
-    else
-        batch_pass_kernel<256><<<b->sm_count * b->cps, 256, batch_smem(b->cps), b->st>>>(
-            b->d_reps, b->d_items, b->nitems, b->d_state, b->k);
+    auto kern = b->cps <= 1 ? (b->general ? batch_pass_kernel<BATCH_THREADS, DEC_ANY> : batch_pass_kernel<BATCH_THREADS, DEC_ANY_FEW>)
+                            : (b->general ? batch_pass_kernel<256, DEC_ANY> : batch_pass_kernel<256, DEC_ANY_FEW>);
+    kern<<<b->sm_count * b->cps, batch_threads(b->cps), batch_smem(b->cps), b->st>>>(b->d_reps, b->d_items, b->nitems,
+                                                                                     b->d_state, b->k);
     batch_advance_kernel<<<1, 1, 0, b->st>>>(b->d_state, b->k);
     return cudaGetLastError();
 }
@@ -243,6 +245,7 @@ extern "C" kpzb_status kpzb_batch_create(kpzb_batch** out, int n, const int* lx,
         r.stream = stream ? stream[i] : 0u;
         r.tp = make_thresh(thresh_b(p[i]));
         r.tq = make_thresh(thresh_b(q[i]));
+        b->general |= r.tp.planes > 4 || r.tq.planes > 4;
         const size_t bytes = (size_t)1 << (2 * lx[i] - 2);
         for (int s = 0; s < 2; ++s)
             if ((e = cudaMalloc(&r.buf[s], bytes)) != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(replica)"));
@@ -254,11 +257,14 @@ extern "C" kpzb_status kpzb_batch_create(kpzb_batch** out, int n, const int* lx,
         return bail(cuda_fail(e, "cudaMalloc(state)"));
     cudaMemset(b->d_state, 0, sizeof(PassState));
     if ((e = analysis_alloc(&b->an, b->max_ly)) != cudaSuccess) return bail(cuda_fail(e, "analysis_alloc"));
-    if ((e = cudaFuncSetAttribute(batch_pass_kernel<BATCH_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)BATCH_SMEM)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(batch_pass_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)batch_smem(2))) != cudaSuccess)
-        return bail(cuda_fail(e, "smem attribute"));
+    auto allow = [&](auto kern, int cps) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_smem(cps));
+    };
+    allow(batch_pass_kernel<BATCH_THREADS, DEC_ANY>, 1);
+    allow(batch_pass_kernel<BATCH_THREADS, DEC_ANY_FEW>, 1);
+    allow(batch_pass_kernel<256, DEC_ANY>, 2);
+    allow(batch_pass_kernel<256, DEC_ANY_FEW>, 2);
+    if (e != cudaSuccess) return bail(cuda_fail(e, "smem attribute"));
     kpzb_status s = batch_layout(b);
     if (s != KPZB_OK) return bail(s);
     s = kpzb_batch_init_homogeneous(b);

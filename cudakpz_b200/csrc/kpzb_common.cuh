@@ -289,7 +289,10 @@ __device__ __forceinline__ uint4 decide4_few(uint4 cp, uint4 cq, Thresh tp, Thre
 //   DEC_GENERAL anything else (bit-serial loop of decide4).
 //   DEC_FEW    DEC_GENERAL's rates of at most four planes, where a kernel has an instance of its own
 //              for them (decide4_few).
-enum DecMode { DEC_NONE = 0, DEC_ONE = 1, DEC_GENERAL = 2, DEC_FEW = 3 };
+// And for kernels whose rates are known only at run time, as in a batch:
+//   DEC_ANY      any of these modes,
+//   DEC_ANY_FEW  any of them but DEC_GENERAL.
+enum DecMode { DEC_ANY_FEW = -2, DEC_ANY = -1, DEC_NONE = 0, DEC_ONE = 1, DEC_GENERAL = 2, DEC_FEW = 3 };
 
 __host__ __device__ inline int dec_mode(Thresh tp, Thresh tq)
 {
@@ -299,7 +302,8 @@ __host__ __device__ inline int dec_mode(Thresh tp, Thresh tq)
 
 // decide4 with the cheap modes spelled out; identical results in every mode.
 // slot: sixteen bytes of shared memory per warp where all 32 lanes call together, else nullptr.
-template <bool WARP = false>
+// GENERAL: false where DEC_GENERAL is not among the caller's modes.
+template <bool WARP = false, bool GENERAL = true>
 __device__ __forceinline__ uint4 decide4_mode(int mode, uint4 cp, uint4 cq, Thresh tp, Thresh tq,
                                               Key key, uint32_t qgroup, uint32_t step,
                                               uint32_t stream, uint8_t* slot = nullptr)
@@ -321,7 +325,7 @@ __device__ __forceinline__ uint4 decide4_mode(int mode, uint4 cp, uint4 cq, Thre
                           (cp.z & (ap | (hp & ~r.z))) | (cq.z & (aq | (hq & ~r.z))),
                           (cp.w & (ap | (hp & ~r.w))) | (cq.w & (aq | (hq & ~r.w))));
     }
-    if (mode == DEC_FEW) return decide4_few(cp, cq, tp, tq, key, qgroup, step, stream);
+    if (!GENERAL || mode == DEC_FEW) return decide4_few(cp, cq, tp, tq, key, qgroup, step, stream);
     return decide4<WARP>(cp, cq, tp, tq, key, qgroup, PlaneMaker{step, key}, stream, slot);
 }
 

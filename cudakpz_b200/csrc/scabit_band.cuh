@@ -141,7 +141,7 @@ __device__ __forceinline__ uint4 sca_decide(const uint4& tX, const uint4& tY, co
                           (cp.w & ap) | (cq.w & aq));
     }
     if (WARP && !live) cp = cq = make_uint4(0, 0, 0, 0);
-    return decide4_mode<WARP>(MODE < 0 ? mode_rt : MODE, cp, cq, tp, tq, key, qgroup, step, stream, slot);
+    return decide4_mode<WARP, MODE != DEC_ANY_FEW>(MODE < 0 ? mode_rt : MODE, cp, cq, tp, tq, key, qgroup, step, stream, slot);
 }
 
 // The update of one group from its loaded words.  Within a half-step a group may be loaded
@@ -215,7 +215,7 @@ __device__ __forceinline__ void sca_update_group(uint32_t* pTX, uint32_t* pTY, u
 
 // Runs one band; returns false (after flagging *err) when the TMA load did not complete in
 // time.  Must be called by all threads of the CTA; NT = blockDim.x.  MODE / USEQ as for
-// sca_update_group (MODE -1 with USEQ true: rates known only at run time, as in a batch).
+// sca_update_group (DEC_ANY and DEC_ANY_FEW with USEQ true).
 template <int MODE, bool USEQ, bool COUNT, int NT>
 __device__ bool scabit_band(uint32_t* smem, const BandCtl& ctl, const BandGeom& g,
                             unsigned long long& ndep, unsigned long long& ndes,
@@ -292,29 +292,39 @@ __device__ bool scabit_band(uint32_t* smem, const BandCtl& ctl, const BandGeom& 
         const int rb = g.resident ? R : R - 1 - h;
         auto update = [&](auto warp_tag, int gg, int lr, bool live) {
             constexpr bool WARP = decltype(warp_tag)::value;
+            constexpr int M = MODE >= 0 ? MODE : WARP ? (int)DEC_GENERAL : (int)DEC_ANY_FEW;
             const uint32_t w0 = 4u * (uint32_t)gg;
             const uint32_t wnext = (w0 + 4u) & (wr - 1u);
             const uint32_t gy = ((uint32_t)ylo32 + (uint32_t)lr) & rmask;  // periodic in y
             const uint32_t ro = (uint32_t)lr * wr;
             const uint32_t ro1 = g.resident ? (((uint32_t)lr + 1u) & rmask) * wr : ro + wr;
-            sca_update_group<MODE, USEQ, COUNT, WARP>(StX + ro + w0, StY + ro + w0, SoX + ro + w0, SoY + ro1 + w0,
-                                                      SoX + ro + wnext, sigma != (int)(gy & 1u), mode_rt, g.tp, g.tq,
-                                                      g.key, (gy << lgG) + (uint32_t)gg, step, g.stream,
-                                                      lr >= H && lr < H + Bc, ndep, ndes, live, slot_s[threadIdx.x >> 5]);
+            sca_update_group<M, USEQ, COUNT, WARP>(StX + ro + w0, StY + ro + w0, SoX + ro + w0, SoY + ro1 + w0,
+                                                   SoX + ro + wnext, sigma != (int)(gy & 1u), mode_rt, g.tp, g.tq,
+                                                   g.key, (gy << lgG) + (uint32_t)gg, step, g.stream,
+                                                   lr >= H && lr < H + Bc, ndep, ndes, live, slot_s[threadIdx.x >> 5]);
         };
-        if (MODE == DEC_GENERAL || (MODE < 0 && mode_rt == DEC_GENERAL)) {
-            // every warp stays together: lanes past the last row repeat a row without effect
-            for (int gg = gi; gg < G; gg += NT)
-                for (int l0 = ra; l0 < rb; l0 += rstride) {
-                    const int lr = l0 + rofs;
-                    update(std::true_type{}, gg, lr < rb ? lr : ra, lr < rb);
-                }
-            __syncthreads();
-            continue;
-        }
         // wide rows (G > NT): a thread takes several column groups of a row in turn
-        for (int gg = gi; gg < G; gg += NT) {
-            for (int lr = ra + rofs; lr < rb; lr += rstride) update(std::false_type{}, gg, lr, true);
+        auto each = [&](auto warp_tag) {
+            constexpr bool WARP = decltype(warp_tag)::value;
+            for (int gg = gi; gg < G; gg += NT) {
+                if constexpr (WARP) {
+                    // every warp stays together: lanes past the last row repeat a row without effect
+                    for (int l0 = ra; l0 < rb; l0 += rstride) {
+                        const int lr = l0 + rofs;
+                        update(warp_tag, gg, lr < rb ? lr : ra, lr < rb);
+                    }
+                } else {
+                    for (int lr = ra + rofs; lr < rb; lr += rstride) update(warp_tag, gg, lr, true);
+                }
+            }
+        };
+        if constexpr (MODE == DEC_GENERAL) {
+            each(std::true_type{});
+        } else if constexpr (MODE == DEC_ANY) {
+            if (mode_rt == DEC_GENERAL) each(std::true_type{});
+            else each(std::false_type{});
+        } else {
+            each(std::false_type{});
         }
         __syncthreads();
     }
