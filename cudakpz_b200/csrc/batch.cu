@@ -78,8 +78,10 @@ batch_pass_kernel(const RepDesc* __restrict__ reps, const Item* __restrict__ ite
     const uint32_t par = st->parity;
     uint32_t phase = 0;
     unsigned long long nd = 0, nr = 0;
-    for (;;) {
-        if (threadIdx.x == 0) cur = (int)atomicAdd(&st->queue, 1u);
+    // A CTA's first item goes by its index, so that fewer items than CTAs spread over the SMs as the
+    // CTAs do instead of falling to those that start first.
+    for (bool first = true;; first = false) {
+        if (threadIdx.x == 0) cur = first ? (int)blockIdx.x : (int)(gridDim.x + atomicAdd(&st->queue, 1u));
         __syncthreads();
         const int i = cur;
         __syncthreads();
@@ -194,8 +196,10 @@ static cudaError_t enqueue_pass(kpzb_batch* b)
 {
     auto kern = b->cps <= 1 ? (b->general ? batch_pass_kernel<BATCH_THREADS, DEC_ANY> : batch_pass_kernel<BATCH_THREADS, DEC_ANY_FEW>)
                             : (b->general ? batch_pass_kernel<256, DEC_ANY> : batch_pass_kernel<256, DEC_ANY_FEW>);
-    kern<<<b->sm_count * b->cps, batch_threads(b->cps), batch_smem(b->cps), b->st>>>(b->d_reps, b->d_items, b->nitems,
-                                                                                     b->d_state, b->k);
+    // no CTA without an item: a grid of all slots fills some SMs before others have their first CTA
+    // (444 CTAs: six SMs get three of the first 148; a grid of 284 leaves two or one on every SM)
+    const int grid = std::min(b->sm_count * b->cps, b->nitems);
+    kern<<<grid, batch_threads(b->cps), batch_smem(b->cps), b->st>>>(b->d_reps, b->d_items, b->nitems, b->d_state, b->k);
     batch_advance_kernel<<<1, 1, 0, b->st>>>(b->d_state, b->k);
     return cudaGetLastError();
 }
