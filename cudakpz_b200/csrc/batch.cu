@@ -125,6 +125,7 @@ struct kpzb_batch {
     int k = 8;                   // MCS per pass
     int chunk = 8;               // passes per graph replay
     int cps = 1;                 // CTAs per SM (1: 512 threads, 2 or 3: 256 threads each)
+    size_t smem = BATCH_SMEM;    // shared memory of a CTA
     bool general = false;        // some replica's rates need more than four random planes
     bool planned = false;        // k and cps set by the caller or the tuner (else tuned on first MCS)
     cudaGraphExec_t graph = nullptr;
@@ -150,12 +151,21 @@ static kpzb_status batch_layout(kpzb_batch* b)
         if (se != cudaSuccess) return cuda_fail(se, "batch sync");
     }
     std::vector<std::pair<double, Item>> work;
+    size_t smem = batch_smem(b->cps);
+    // Where that holds no output row beside the halo (4096^2 at two CTAs per SM, 28 MCS per pass), the
+    // kilobyte kept for static shared memory does; one CTA fewer then fits on an SM.
+    if (b->cps > 1)
+        for (const RepDesc& r : b->reps)
+            if ((16ull << (2 * r.lx - 6)) > smem && (int64_t)(smem >> (r.lx - 2)) <= 4 * b->k) {
+                smem += 1024;
+                break;
+            }
+    b->smem = smem;
     for (int i = 0; i < b->n; ++i) {
         RepDesc& r = b->reps[i];
         const uint64_t Wr = 1ull << (r.lx - 6);
         const uint64_t row_bytes = 16ull * Wr;
         const int64_t rows = 1ll << r.ly;
-        const size_t smem = batch_smem(b->cps);
         if ((uint64_t)rows * row_bytes <= smem) {
             r.resident = 1;
             r.B = (int)rows;
@@ -199,7 +209,7 @@ static cudaError_t enqueue_pass(kpzb_batch* b)
     // no CTA without an item: a grid of all slots fills some SMs before others have their first CTA
     // (444 CTAs: six SMs get three of the first 148; a grid of 284 leaves two or one on every SM)
     const int grid = std::min(b->sm_count * b->cps, b->nitems);
-    kern<<<grid, batch_threads(b->cps), batch_smem(b->cps), b->st>>>(b->d_reps, b->d_items, b->nitems, b->d_state, b->k);
+    kern<<<grid, batch_threads(b->cps), b->smem, b->st>>>(b->d_reps, b->d_items, b->nitems, b->d_state, b->k);
     batch_advance_kernel<<<1, 1, 0, b->st>>>(b->d_state, b->k);
     return cudaGetLastError();
 }
@@ -261,13 +271,13 @@ extern "C" kpzb_status kpzb_batch_create(kpzb_batch** out, int n, const int* lx,
         return bail(cuda_fail(e, "cudaMalloc(state)"));
     cudaMemset(b->d_state, 0, sizeof(PassState));
     if ((e = analysis_alloc(&b->an, b->max_ly)) != cudaSuccess) return bail(cuda_fail(e, "analysis_alloc"));
-    auto allow = [&](auto kern, int cps) {
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_smem(cps));
+    auto allow = [&](auto kern, size_t smem) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     };
-    allow(batch_pass_kernel<BATCH_THREADS, DEC_ANY>, 1);
-    allow(batch_pass_kernel<BATCH_THREADS, DEC_ANY_FEW>, 1);
-    allow(batch_pass_kernel<256, DEC_ANY>, 2);
-    allow(batch_pass_kernel<256, DEC_ANY_FEW>, 2);
+    allow(batch_pass_kernel<BATCH_THREADS, DEC_ANY>, BATCH_SMEM);
+    allow(batch_pass_kernel<BATCH_THREADS, DEC_ANY_FEW>, BATCH_SMEM);
+    allow(batch_pass_kernel<256, DEC_ANY>, batch_smem(2) + 1024);
+    allow(batch_pass_kernel<256, DEC_ANY_FEW>, batch_smem(2) + 1024);
     if (e != cudaSuccess) return bail(cuda_fail(e, "smem attribute"));
     kpzb_status s = batch_layout(b);
     if (s != KPZB_OK) return bail(s);

@@ -1,6 +1,6 @@
 """Batch passes with fewer work items than CTAs, as many, and more, at every number of CTAs per SM,
 in batches without and with rates of more than four random planes: every replica equals the
-oracle."""
+oracle.  The deepest pass that a lattice row fits in a CTA's shared memory, and the one beyond it."""
 import numpy as np
 import pytest
 
@@ -22,4 +22,21 @@ def test_items_and_modes(kpzb, oracle, lxs, general, cps):
         ref = oracle.homogeneous(lxs[i], lxs[i], oracle.ENC_CBBIT)
         oracle.sca_mcs_words(ref, lxs[i], lxs[i], 40 + i, 0, 0, n, *pq[i])
         assert np.array_equal(b.pop(i), ref), (i, lxs[i], pq[i])
+    b.close()
+
+
+@pytest.mark.parametrize("lx,cps,k", [(12, 2, 28), (13, 2, 13), (12, 3, 18), (13, 3, 9), (14, 3, 4)])
+def test_deepest_pass(kpzb, oracle, lx, cps, k):
+    b = kpzb.Batch([lx, 8], [1.0, 0.5], [0.0, 0.5], [3, 4])
+    b.setFusion(k)  # the default depth of 8 does not fit every row below
+    b.setCtasPerSm(cps)
+    with pytest.raises(kpzb.KpzbError) as e:
+        b.setFusion(k + 1)
+    assert e.value.status == 1
+    b.setFusion(k)
+    b.mcs(k)
+    for i, (l, p, q) in enumerate([(lx, 1.0, 0.0), (8, 0.5, 0.5)]):
+        ref = oracle.homogeneous(l, l, oracle.ENC_CBBIT)
+        oracle.sca_mcs_words(ref, l, l, 3 + i, 0, 0, k, p, q)
+        assert np.array_equal(b.pop(i), ref)
     b.close()
