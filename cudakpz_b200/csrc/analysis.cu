@@ -35,9 +35,16 @@ struct Partial {
     double pad2[3];
 };
 
-// Per-row record {n1, n2, n3, w}: the X-slope bits set in the row's first one, two and three
-// quarters (rows of at least AN_PART_WORDS words; else 0), and w = x-slope row sum (even) with the
-// y-slope bit of x = 0 in bit 0.
+// Per-row record w: x-slope row sum (even) with the y-slope bit of x = 0 in bit 0.  Rows of at least
+// AN_PART_WORDS words have {n1, n2, n3, w} with the X-slope bits set in the row's first one, two and
+// three quarters; the others only w, since tall lattices have many of them (4 bytes a row instead of
+// 16 are 24 GiB of a lattice of 2^8 x 2^30).
+__host__ __device__ constexpr bool long_rows(int lx) { return (1ull << lx) >= 64ull * AN_PART_WORDS; }
+__host__ __device__ constexpr int row_ints(int lx) { return long_rows(lx) ? 4 : 1; }
+__device__ __forceinline__ int row_word(const int* rowinfo, uint64_t y, int lx)
+{
+    return rowinfo[(y + 1) * row_ints(lx) - 1];
+}
 __device__ __forceinline__ int row_sum(int w) { return w & ~1; }
 __device__ __forceinline__ int row_ystep(int w) { return 2 * (w & 1) - 1; }
 
@@ -105,7 +112,7 @@ __device__ __forceinline__ uint4 load_words4(const uint32_t* p)
 template <bool WORDS>
 __global__ void __launch_bounds__(AN_ROW_THREADS)
 row_kernel(const uint32_t* __restrict__ sys0, const uint32_t* __restrict__ sys1, int lx, int ly,
-           int4* __restrict__ rowinfo0, int64_t* __restrict__ rowstart0, WalkState* ws)
+           int* __restrict__ rowinfo0, int64_t* __restrict__ rowstart0, WalkState* ws)
 {
     __shared__ int w_s[AN_ROW_THREADS];
     __shared__ long long lo_s[AN_ROW_THREADS / 32], hi_s[AN_ROW_THREADS / 32];
@@ -113,7 +120,7 @@ row_kernel(const uint32_t* __restrict__ sys0, const uint32_t* __restrict__ sys1,
     const uint64_t Q = 1ull << (lx + ly - 6);
     const uint64_t rows = 1ull << ly;
     const uint32_t* sys = blockIdx.y ? sys1 : sys0;
-    int4* rowinfo = rowinfo0 + blockIdx.y * rows;
+    int* rowinfo = rowinfo0 + blockIdx.y * rows * row_ints(lx);
     int64_t* rowstart = rowstart0 + blockIdx.y * rows;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     constexpr int NWARP = AN_ROW_THREADS / 32;
@@ -129,7 +136,8 @@ row_kernel(const uint32_t* __restrict__ sys0, const uint32_t* __restrict__ sys1,
         const uint64_t end = ye - base < AN_ROW_THREADS ? ye : base + AN_ROW_THREADS;
         auto put = [&](uint64_t y, int n1, int n2, int n3, int n, int s) {
             const int w = (int)(2 * (int64_t)n - (int64_t)(1ull << lx)) | s;
-            rowinfo[y] = make_int4(n1, n2, n3, w);
+            if (long_rows(lx)) reinterpret_cast<int4*>(rowinfo)[y] = make_int4(n1, n2, n3, w);
+            else rowinfo[y] = w;
             w_s[y - base] = w;
         };
         if (Wr >= AN_PART_WORDS) {
@@ -345,7 +353,7 @@ __device__ __forceinline__ Partial empty_partial()
 // them where rows are long.
 struct WalkGeom {
     const uint32_t *sys, *snap;
-    const int4* rowinfo;      // of the system; the snapshot's 2^ly further on
+    const int* rowinfo;       // records of the system's rows, then of the snapshot's
     const int64_t* rowstart;
     const long long *base, *base_s;  // heights at the start of every row block
     const uint32_t* step4;           // table of add_chunk
@@ -414,16 +422,19 @@ __device__ __forceinline__ void walk_chunks(const WalkGeom& g, F&& chunk)
         };
         load(sub);
         // height before the part's first site: Hs - e0 + 2 (bits set before it) - sites
+        auto record = [&](uint64_t i) {
+            return parts > 1 ? reinterpret_cast<const int4*>(g.rowinfo)[i] : make_int4(0, 0, 0, g.rowinfo[i]);
+        };
         auto before = [&](const int4& r) { return part == 0 ? 0 : part == 1 ? r.x : part == 2 ? r.y : r.z; };
         const long long back = (long long)(64 * pw * part);
-        const int4 ri = g.rowinfo[y];
+        const int4 ri = record(y);
         long long H = g.rowstart[y] + g.base[y >> lgb] - (2 * (int)(g.sys[be + y * Wr] & 1u) - 1) +
                       2 * (long long)before(ri) - back - g.mid;
         long long Hsn = 0;
         Chunk ch{};
         ch.sum_r = row_sum(ri.w);
         if (CORR) {
-            const int4 si = g.rowinfo[rows + y];
+            const int4 si = record(rows + y);
             ch.sum_s = row_sum(si.w);
             Hsn = g.rowstart[rows + y] + g.base_s[y >> lgb] - (2 * (int)(g.snap[be + y * Wr] & 1u) - 1) +
                   2 * (long long)before(si) - back - g.mid_s;
@@ -590,7 +601,7 @@ constexpr int walk_threads(bool corr) { return corr ? 768 : 1024; }  // 85 and 6
 template <bool CORR>
 __global__ void __launch_bounds__(walk_threads(CORR), 1)
 walk_kernel(const uint32_t* __restrict__ sys, const uint32_t* __restrict__ snap, int lx, int ly,
-            const int4* __restrict__ rowinfo, const int64_t* __restrict__ rowstart, Partial* __restrict__ partials,
+            const int* __restrict__ rowinfo, const int64_t* __restrict__ rowstart, Partial* __restrict__ partials,
             Partial* __restrict__ out, WalkState* ws)
 {
     constexpr int NT = walk_threads(CORR), NWARP = NT / 32;
@@ -813,7 +824,7 @@ walk_kernel(const uint32_t* __restrict__ sys, const uint32_t* __restrict__ snap,
 
 // {Hs(y) - c, h(0, y) - c} of every row, from the row tables of the lattice measured last.
 __global__ void __launch_bounds__(AN_ROW_THREADS)
-row_heights_kernel(const int4* __restrict__ rowinfo, const int64_t* __restrict__ rowstart, int ly, int64_t c,
+row_heights_kernel(const int* __restrict__ rowinfo, const int64_t* __restrict__ rowstart, int lx, int ly, int64_t c,
                    const WalkState* __restrict__ ws, int2* __restrict__ out)
 {
     __shared__ long long base_s[AN_MAX_BLOCKS];
@@ -822,17 +833,17 @@ row_heights_kernel(const int4* __restrict__ rowinfo, const int64_t* __restrict__
     row_block_bases<AN_ROW_THREADS>(ws->block[0], (int)(rows >> lgb), base_s);
     for (uint64_t y = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; y < rows; y += (uint64_t)gridDim.x * blockDim.x) {
         const int64_t h = rowstart[y] + base_s[y >> lgb] - c;
-        out[y] = make_int2((int32_t)h, (int32_t)(h + row_sum(rowinfo[y].w)));
+        out[y] = make_int2((int32_t)h, (int32_t)(h + row_sum(row_word(rowinfo, y, lx))));
     }
 }
 
-cudaError_t analysis_alloc(AnalysisScratch* s, int ly)
+cudaError_t analysis_alloc(AnalysisScratch* s, int lx, int ly)
 {
     const size_t rows = 1ull << ly;
     s->rows_cap = rows;
     cudaError_t e;
     // two row tables (system and snapshot) and partials, final record and the walk's state
-    if ((e = cudaMalloc(&s->rowinfo, 2 * rows * sizeof(int4))) != cudaSuccess) return e;
+    if ((e = cudaMalloc(&s->rowinfo, 2 * rows * row_ints(lx) * sizeof(int))) != cudaSuccess) return e;
     if ((e = cudaMalloc(&s->rowstart, 2 * rows * sizeof(int64_t))) != cudaSuccess) return e;
     const size_t acc = (AN_MAX_GRID + 1) * sizeof(Partial) + sizeof(WalkState);
     return cudaMalloc(&s->acc, acc);
@@ -896,11 +907,11 @@ cudaError_t analysis_moments_record(const uint32_t* d_sys, const uint32_t* d_sna
     return cudaGetLastError();
 }
 
-cudaError_t analysis_row_heights(AnalysisScratch* s, int ly, int64_t c, int2* d_out, cudaStream_t st)
+cudaError_t analysis_row_heights(AnalysisScratch* s, int lx, int ly, int64_t c, int2* d_out, cudaStream_t st)
 {
     const uint64_t rows = 1ull << ly;
     const unsigned grid = (unsigned)(rows / AN_ROW_THREADS < 592 ? rows / AN_ROW_THREADS + 1 : 592);
-    row_heights_kernel<<<grid, AN_ROW_THREADS, 0, st>>>(s->rowinfo, s->rowstart, ly, c, walk_state(s), d_out);
+    row_heights_kernel<<<grid, AN_ROW_THREADS, 0, st>>>(s->rowinfo, s->rowstart, lx, ly, c, walk_state(s), d_out);
     return cudaGetLastError();
 }
 
@@ -951,7 +962,7 @@ __global__ void colsum_kernel(const uint32_t* __restrict__ sys, int lx, int ly, 
 }
 
 __global__ void invariants_kernel(const uint32_t* __restrict__ sys, int lx, int ly,
-                                  const int4* __restrict__ rowinfo, const int* __restrict__ colsum,
+                                  const int* __restrict__ rowinfo, const int* __restrict__ colsum,
                                   unsigned long long* rep)
 {
     const uint64_t Wr = 1ull << (lx - 6);
@@ -961,7 +972,7 @@ __global__ void invariants_kernel(const uint32_t* __restrict__ sys, int lx, int 
     unsigned long long badr = 0, badc = 0, badp = 0;
     const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t y = tid; y < rows; y += nth) badr += row_sum(rowinfo[y].w) != 0;
+    for (uint64_t y = tid; y < rows; y += nth) badr += row_sum(row_word(rowinfo, y, lx)) != 0;
     for (uint64_t x = tid; x < L; x += nth) badc += colsum[x] != 0;
     // plaquettes: per (sublattice, row, word)
     for (uint64_t i = tid; i < 2 * Q; i += nth) {
@@ -1132,7 +1143,7 @@ extern "C" kpzb_status kpzb_roughness_noalloc(const uint32_t* d_cbbit, int lx, i
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(no-alloc scratch)");
     unsigned char* base = static_cast<unsigned char*>(addr);
     AnalysisScratch view;
-    view.rowinfo = reinterpret_cast<int4*>(base);
+    view.rowinfo = reinterpret_cast<int*>(base);
     view.rowstart = reinterpret_cast<int64_t*>(base + NOALLOC_ROWINFO);
     view.acc = reinterpret_cast<unsigned long long*>(base + NOALLOC_ROWINFO + NOALLOC_ROWSTART);
     view.rows_cap = 1ull << NOALLOC_MAX_LY;

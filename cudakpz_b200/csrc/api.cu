@@ -155,7 +155,7 @@ extern "C" kpzb_status kpzb_create(kpzb_handle** out, int lx, int ly, int dynami
     if ((e = cudaMalloc(&h->d_counters, 4 * sizeof(unsigned long long))) != cudaSuccess)
         return bail(cuda_fail(e, "cudaMalloc(counters)"));
     cudaMemsetAsync(h->d_counters, 0, 4 * sizeof(unsigned long long), h->st);
-    if ((e = analysis_alloc(&h->an, ly)) != cudaSuccess) return bail(cuda_fail(e, "analysis_alloc"));
+    if ((e = analysis_alloc(&h->an, lx, ly)) != cudaSuccess) return bail(cuda_fail(e, "analysis_alloc"));
     if (h->rs()) {
         kpzb_status s = dt_init(&h->dt, lx, ly, h->sm_count, dynamics == KPZB_DYN_DB4);
         if (s != KPZB_OK) return bail(s);

@@ -270,7 +270,7 @@ extern "C" kpzb_status kpzb_batch_create(kpzb_batch** out, int n, const int* lx,
     if ((e = cudaMalloc(&b->d_state, sizeof(PassState))) != cudaSuccess)
         return bail(cuda_fail(e, "cudaMalloc(state)"));
     cudaMemset(b->d_state, 0, sizeof(PassState));
-    if ((e = analysis_alloc(&b->an, b->max_ly)) != cudaSuccess) return bail(cuda_fail(e, "analysis_alloc"));
+    if ((e = analysis_alloc(&b->an, b->max_ly, b->max_ly)) != cudaSuccess) return bail(cuda_fail(e, "analysis_alloc"));
     auto allow = [&](auto kern, size_t smem) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     };

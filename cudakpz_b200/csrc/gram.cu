@@ -158,7 +158,7 @@ extern "C" kpzb_status kpzb_gram_create(kpzb_gram** out, int lx, int ly, int max
     if ((e = cudaMalloc(&g->d_rows, (size_t)max_snapshots * g->rows * sizeof(int2))) != cudaSuccess)
         return bail(cuda_fail(e, "cudaMalloc(snapshot rows)"));
     if ((e = cudaMalloc(&g->d_g, 64 * 64 * 8)) != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(G)"));
-    if ((e = analysis_alloc(&g->an, ly)) != cudaSuccess) return bail(cuda_fail(e, "analysis_alloc"));
+    if ((e = analysis_alloc(&g->an, lx, ly)) != cudaSuccess) return bail(cuda_fail(e, "analysis_alloc"));
     kpzb_status s = gram_tc_setup(&g->tc, g->N, g->sm_count);
     if (s != KPZB_OK) return bail(s);
     *out = g;
@@ -201,7 +201,7 @@ extern "C" kpzb_status kpzb_gram_add_device(kpzb_gram* g, const uint32_t* d_cbbi
     gram_store_kernel<<<grid, 256, 0, g->st>>>(d_cbbit, g->Q, g->smax, s, reinterpret_cast<uint4*>(g->d_snap));
     GCU(cudaGetLastError(), "gram_store_kernel");
     // per-row data {b(y), z(y)} = {Hs(y) - c, h(0, y) - c}
-    GCU(analysis_row_heights(&g->an, g->ly, c, g->d_rows + (uint64_t)s * g->rows, g->st), "snapshot rows");
+    GCU(analysis_row_heights(&g->an, g->lx, g->ly, c, g->d_rows + (uint64_t)s * g->rows, g->st), "snapshot rows");
     GCU(cudaStreamSynchronize(g->st), "snapshot sync");
     g->vmin = std::min<int64_t>(g->vmin, m.hmin - c);
     g->vmax = std::max<int64_t>(g->vmax, m.hmax - c);

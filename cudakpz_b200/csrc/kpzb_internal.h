@@ -101,12 +101,12 @@ cudaError_t cbbit_to_local_dev(const uint32_t* cbbit, uint32_t* local, int lx, i
 
 // analysis on ENC_CBBIT lattices
 struct AnalysisScratch {
-    int4* rowinfo;         // 2 * rows (system, snapshot): slope counts of each row (see analysis.cu)
+    int* rowinfo;          // 2 * rows (system, snapshot): slope counts of each row (see analysis.cu)
     int64_t* rowstart;     // 2 * rows: height at the start of each row walk, within its row block
     unsigned long long* acc;  // partial sums and the walk's state (see analysis.cu)
     size_t rows_cap;
 };
-cudaError_t analysis_alloc(AnalysisScratch* s, int ly);
+cudaError_t analysis_alloc(AnalysisScratch* s, int lx, int ly);  // for lattices up to that wide and tall
 void analysis_free(AnalysisScratch* s);
 // out_i64[0..2]: S1, S2, hmin/hmax packed; out_f64[0..4]: S3..S7; corr outputs optional
 struct MomentsOut {
@@ -128,7 +128,7 @@ cudaError_t analysis_moments_record(const uint32_t* d_sys, const uint32_t* d_sna
 void analysis_decode_record(const void* rec, MomentsOut* out);
 // {Hs(y) - c, h(0, y) - c} of every row of the lattice measured last with s (Hs: the height the
 // walk carries into row y) into d_out[2^ly]
-cudaError_t analysis_row_heights(AnalysisScratch* s, int ly, int64_t c, int2* d_out, cudaStream_t st);
+cudaError_t analysis_row_heights(AnalysisScratch* s, int lx, int ly, int64_t c, int2* d_out, cudaStream_t st);
 // invariants: rep[0] bad rows, rep[1] bad columns, rep[2] bad plaquettes
 cudaError_t analysis_invariants(const uint32_t* d_sys, int lx, int ly, AnalysisScratch* s,
                                 int64_t rep[3], cudaStream_t st);
