@@ -201,7 +201,7 @@ struct DtSite {
         }
     }
     template <bool COUNT>
-    __device__ __forceinline__ void flip(uint32_t u, const DtRule& rule, const DisorderRates& dr,
+    __device__ __forceinline__ void flip(uint32_t u, const DtRule& rule, const uint2* rates,
                                          unsigned long long& ndep, unsigned long long& ndes) const
     {
         // bit 0 (bit 1): x-slope of the site (of its right neighbour); bit 0 of ys, yd: y-slope of the
@@ -212,9 +212,9 @@ struct DtSite {
         const bool is_q = (xs & 1u) != 0u;
         bool ok;
         if (DIS) {
-            const int cls = (int)((__funnelshift_r(d0, d0, x) & 1u) | ((__funnelshift_r(d1, d1, x) & 1u) << 1));
-            const Thresh& th = is_q ? dr.tq[cls] : dr.tp[cls];
-            ok = th.always || (th.planes && u < th.t);
+            const uint32_t cls = (__funnelshift_r(d0, d0, x) & 1u) | ((__funnelshift_r(d1, d1, x) & 1u) << 1);
+            const uint2 r = rates[2u * cls + (is_q ? 1u : 0u)];
+            ok = r.x && u <= r.y;
         } else {
             ok = (is_q ? rule.ok_q : rule.ok_p) && u <= (is_q ? rule.lim_q : rule.lim_p);
         }
@@ -281,6 +281,11 @@ dt_scatter_kernel(uint32_t* __restrict__ sys, int lxw, int lyw, int lnbx, int ox
     __shared__ uint32_t plane[(DIS ? 4 : 2) * PL_WORDS];
     __shared__ uint32_t hits_s[REP ? WARPS : 1];
     __shared__ uint32_t need_s[3];
+    // rate classes: {whether a deposition (desorption) candidate can flip, its acceptance limit}; as
+    // a kernel parameter indexed by lane the thresholds went through local memory (four classes with
+    // counters at 8192^2: DTDBSH 460 -> 330 us a MCS, DBSH 635 -> 445; two classes at 16384^2: DBSH
+    // 1650 -> 1380)
+    __shared__ uint2 rate_s[DIS ? 8 : 1];
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t Wx = 1u << lxw, Wy = 1u << lyw;
     const uint32_t ax = ox & 3, ay = oy & 3;
@@ -296,6 +301,14 @@ dt_scatter_kernel(uint32_t* __restrict__ sys, int lxw, int lyw, int lnbx, int ox
     planes_load(sys, plane, tid, NT, wx0, wy0, Wx, Wy);
     if (DIS) planes_load(dis, plane + 2 * PL_WORDS, tid, NT, wx0, wy0, Wx, Wy);
     if (tid < 3) need_s[tid] = 0u;
+    if (DIS && tid == 0) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const DtRule r = make_rule(dr.tp[c], dr.tq[c]);
+            rate_s[2 * c] = make_uint2(r.ok_p, r.lim_p);
+            rate_s[2 * c + 1] = make_uint2(r.ok_q, r.lim_q);
+        }
+    }
     __syncthreads();
 
     const int row0 = warp * ROWS;
@@ -366,7 +379,7 @@ dt_scatter_kernel(uint32_t* __restrict__ sys, int lxw, int lyw, int lnbx, int ox
                     if ((go[i] >> (8 * j + 7)) & 1u) site(i, j, s[i]);
 #pragma unroll
                 for (int i = 0; i < ROWS; ++i)
-                    if ((go[i] >> (8 * j + 7)) & 1u) s[i].template flip<COUNT>(pick4(uu[i], j), rule, dr, ndep, ndes);
+                    if ((go[i] >> (8 * j + 7)) & 1u) s[i].template flip<COUNT>(pick4(uu[i], j), rule, rate_s, ndep, ndes);
                 __syncthreads();
                 if (skip_border) continue;
                 if (j == 0) waits = *need;
@@ -379,7 +392,7 @@ dt_scatter_kernel(uint32_t* __restrict__ sys, int lxw, int lyw, int lnbx, int ox
                         if (((late[i] >> (8 * j + 7)) & 1u) && corner == (phase == 2)) {
                             DtSite<DIS> s1;
                             site(i, j, s1);
-                            s1.template flip<COUNT>(pick4(uu[i], j), rule, dr, ndep, ndes);
+                            s1.template flip<COUNT>(pick4(uu[i], j), rule, rate_s, ndep, ndes);
                         }
                     }
                     __syncthreads();
@@ -500,7 +513,7 @@ dt_scatter_kernel(uint32_t* __restrict__ sys, int lxw, int lyw, int lnbx, int ox
                     s[i].load(plane, x, y * (4 * PL_W) + ((x >> 3) & 0x7Cu));
                 }
 #pragma unroll
-                for (int i = 0; i < ROWS; ++i) s[i].template flip<COUNT>(pick4(uu[i], j), rule, dr, ndep, ndes);
+                for (int i = 0; i < ROWS; ++i) s[i].template flip<COUNT>(pick4(uu[i], j), rule, rate_s, ndep, ndes);
                 __syncthreads();
             }
         }
