@@ -263,7 +263,7 @@ __device__ __forceinline__ uint32_t not_adjacent(uint32_t pos, uint32_t right, u
 // order.  That takes one attempt's instructions and 1.8 barriers per round instead of 2.4 and 3.
 // Columns, rows and word offsets of four rounds are formed as bytes of one word.  Measured on a
 // B200, DBSH at p = 0.95, q = 0.05: 16384^2 1592 -> 1248 us per MCS, 1024^2 181 -> 156 us (a launch
-// there is 8 blocks, 64 rounds one after the other); DBSHRep 1583 -> 1239, DTDBSH 929 -> 806 us at
+// there is 8 blocks, 64 rounds one after the other); DBSHRep 1583 -> 1239, DTDBSH 929 -> 779 us at
 // 16384^2.  The integer ALU bounds it.
 //
 // WARPS warps share a block; each owns DT_CY / WARPS cell rows, a cell column per lane, and loads a
@@ -282,9 +282,8 @@ dt_scatter_kernel(uint32_t* __restrict__ sys, int lxw, int lyw, int lnbx, int ox
     __shared__ uint32_t hits_s[REP ? WARPS : 1];
     __shared__ uint32_t need_s[3];
     // rate classes: {whether a deposition (desorption) candidate can flip, its acceptance limit}; as
-    // a kernel parameter indexed by lane the thresholds went through local memory (four classes with
-    // counters at 8192^2: DTDBSH 460 -> 330 us a MCS, DBSH 635 -> 445; two classes at 16384^2: DBSH
-    // 1650 -> 1380)
+    // a kernel parameter indexed by lane the thresholds went through local memory (DBSH, four classes
+    // with counters at 8192^2: 635 -> 444 us a MCS; two classes at 16384^2: 1651 -> 1383)
     __shared__ uint2 rate_s[DIS ? 8 : 1];
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t Wx = 1u << lxw, Wy = 1u << lyw;
@@ -476,41 +475,48 @@ dt_scatter_kernel(uint32_t* __restrict__ sys, int lxw, int lyw, int lnbx, int ox
             }
         }
     } else {
-        // block-wide quadrant sequence: 2 bits per round (every thread derives the same words)
+        // BaseDTInnerDTDBSH (kpz/kpzSimulationPrimitivesTemplates_BaseInnerDTr.cu:30-85): a
+        // quadrant of the cells and a block-wide offset in [0,8)^2 per round, the site wrapped inside
+        // the block before the origin's in-word offset is added; neighbouring cells' sites stay 4 or
+        // more sites apart.  Quadrants (2 bits per round; every thread derives the same words) and
+        // offsets of four rounds lie in the bytes of one word, as do the wrapped columns and rows.
         uint4 sub = draw((uint32_t)b, TAG_DT_SUB, 0u);
         uint4 ow = make_uint4(0u, 0u, 0u, 0u), pw[ROWS];
         uint32_t sw = 0, pos[ROWS];
+        uint32_t* const first = plane + ay * PL_W;
 #pragma unroll 1
         for (int q = 0; q < DT_ROUNDS / 4; ++q) {
             if ((q & 3) == 0) {
                 sw = next(sub);
                 ow = draw((uint32_t)b, TAG_DBSH_ORIGIN, q >> 2);
             }
+            const uint32_t ob4 = next(ow);
+            uint32_t sc4 = sw & 0xFFu;
+            sw >>= 8;
+            sc4 = (sc4 | (sc4 << 12)) & 0x000F000Fu;
+            sc4 = (sc4 | (sc4 << 6)) & 0x03030303u;
+            const uint32_t sx = ((sc4 & 0x01010101u) << 2) + (ob4 & 0x07070707u);
+            const uint32_t sy = ((sc4 & 0x02020202u) << 1) + ((ob4 >> 3) & 0x07070707u);
             uint4 uu[ROWS];
+            uint32_t xb[ROWS], yb[ROWS];
 #pragma unroll
             for (int i = 0; i < ROWS; ++i) {
                 if ((q & 7) == 0) pw[i] = draw(cid0 + 32u * i, TAG_DT_POS, q >> 3);
                 pos[i] = (q & 1) ? pos[i] >> 16 : next(pw[i]);
                 uu[i] = need_u ? draw(cid0 + 32u * i, TAG_DT, q) : make_uint4(0u, 0u, 0u, 0u);
+                // positions of four rounds, a nibble each (x in bits 0-1, y in bits 2-3), to bytes
+                uint32_t p = __byte_perm(pos[i], 0u, 0x4140);
+                p = (p | (p << 4)) & 0x0F0F0F0Fu;
+                xb[i] = add_bytes(bytes4(cx), (p & 0x03030303u) + sx);
+                yb[i] = (bytes4(cy + 8u * i) + (p >> 2 & 0x03030303u) + sy) & 0x7F7F7F7Fu;
             }
-            const uint32_t ob4 = next(ow);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const uint32_t sc = sw & 3u;
-                sw >>= 2;
-                // BaseDTInnerDTDBSH (kpz/kpzSimulationPrimitivesTemplates_BaseInnerDTr.cu:30-85): the
-                // quadrant and a block-wide offset in [0,8)^2 per round, the site wrapped inside the
-                // block before the origin's in-word offset is added; neighbouring cells' sites stay
-                // 4 or more sites apart
-                const uint32_t ob = ob4 >> (8 * j);
-                const uint32_t sx = cx + 4u * (sc & 1u) + (ob & 7u), sy = cy + 2u * (sc & 2u) + ((ob >> 3) & 7u);
                 DtSite<DIS> s[ROWS];
 #pragma unroll
                 for (int i = 0; i < ROWS; ++i) {
-                    const uint32_t p = pos[i] >> (4 * j);
-                    const uint32_t x = ((sx + (p & 3u)) & (DT_BX - 1)) + ax;
-                    const uint32_t y = ((sy + 8u * i + ((p >> 2) & 3u)) & (DT_BY - 1)) + ay;
-                    s[i].load(plane, x, y * (4 * PL_W) + ((x >> 3) & 0x7Cu));
+                    const uint32_t x = __byte_perm(xb[i], 0u, 0x4440 | j) + ax;
+                    s[i].load(first, x, __byte_perm(yb[i], 0u, 0x4440 | j) * (4 * PL_W) + ((x >> 3) & 0x7Cu));
                 }
 #pragma unroll
                 for (int i = 0; i < ROWS; ++i) s[i].template flip<COUNT>(pick4(uu[i], j), rule, rate_s, ndep, ndes);
@@ -713,7 +719,9 @@ dt_quadrant_kernel(uint32_t* __restrict__ sys, int lxw, int lyw, int lnbx, int n
 
 // Warps of a scattered-site block: eight (two cell rows each) where the blocks fill the SMs, else
 // sixteen, whose rounds are shortest.  DBSH at 16384^2 (2048 blocks a launch): 8 warps 1247 us per
-// MCS, 16 warps 1420, 4 warps 1311; at 4096^2 (128 blocks): 16 warps 158 us, 8 warps 197.
+// MCS, 16 warps 1420, 4 warps 1311; at 8192^2 (512): 8 warps 397, 16 warps 432; at 8192 x 4096 (256):
+// 16 warps 232, 8 warps 250; at 4096^2 (128): 16 warps 158 us, 8 warps 197.  DTDBSH at 256 blocks: 150
+// either way.
 constexpr int DT_WARPS_MANY = 8, DT_WARPS_FEW = 16;
 
 // Host copy of the Philox4x32-10 bijection for the per-MCS origin and domain-set order (and
