@@ -49,7 +49,8 @@ constexpr int DT_CELLS = DT_CX * DT_CY;
 constexpr int DT_ROUNDS = 64;
 
 // Philox key schedule by value: every round key is then a constant-bank operand of the round's
-// three-input XOR (3 % to 6 % of these kernels' time; no difference to the SCABit kernels).
+// three-input XOR (3 % to 6 % of these kernels' time where an attempt draws its acceptance; no
+// difference to the SCABit kernels).
 struct DtKey {
     uint32_t k0[10], k1[10];
 };
@@ -644,7 +645,10 @@ dt_quadrant_kernel(uint32_t* __restrict__ sys, int lxw, int lyw, int lnbx, int n
         const uint32_t cid = (uint32_t)b * DT_THREADS + (uint32_t)tid;
         __syncthreads();
         uint4 pos = make_uint4(0, 0, 0, 0), uu = make_uint4(0, 0, 0, 0);
-#pragma unroll 4
+        // all rounds unrolled: four batches at a time the plain instance spilled 24 bytes and the counting
+        // one 40 under the 32 registers of four CTAs per SM (16384^2, p = 1, q = 0: 559 us a MCS,
+        // counting 627; now 532 and 591; at p = 0.95, q = 0.05: 720 -> 682)
+#pragma unroll
         for (int rb = 0; rb < ROUNDS; rb += 8) {
             if ((rb & 31) == 0)
                 pos = philox_dt(
