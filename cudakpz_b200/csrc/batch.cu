@@ -57,7 +57,7 @@ struct PassState {
     uint32_t err;     // set when a bounded wait expired
 };
 
-// MODE: DEC_ANY, or DEC_ANY_FEW for batches whose rates need at most four random planes: the code
+// MODE: DEC_ANY, or DEC_ANY_FEW for batches whose rates need at most three random planes: the code
 // of the general decision costs the others a tenth of their time in registers (8 replicas of 2048^2
 // at (0.75,0.25): 19.2 against 17.4 us a MCS).
 template <int THREADS, int MODE>
@@ -126,7 +126,7 @@ struct kpzb_batch {
     int chunk = 8;               // passes per graph replay
     int cps = 1;                 // CTAs per SM (1: 512 threads, 2 or 3: 256 threads each)
     size_t smem = BATCH_SMEM;    // shared memory of a CTA
-    bool general = false;        // some replica's rates need more than four random planes
+    bool general = false;        // some replica's rates need the general decision
     bool planned = false;        // k and cps set by the caller or the tuner (else tuned on first MCS)
     cudaGraphExec_t graph = nullptr;
     AnalysisScratch an{};
@@ -259,7 +259,7 @@ extern "C" kpzb_status kpzb_batch_create(kpzb_batch** out, int n, const int* lx,
         r.stream = stream ? stream[i] : 0u;
         r.tp = make_thresh(thresh_b(p[i]));
         r.tq = make_thresh(thresh_b(q[i]));
-        b->general |= r.tp.planes > 4 || r.tq.planes > 4;
+        b->general |= dec_mode_few(r.tp, r.tq) == DEC_GENERAL;
         const size_t bytes = (size_t)1 << (2 * lx[i] - 2);
         for (int s = 0; s < 2; ++s)
             if ((e = cudaMalloc(&r.buf[s], bytes)) != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(replica)"));

@@ -235,9 +235,12 @@ __device__ __forceinline__ uint4 decide4(uint4 cp, uint4 cq, Thresh tp, Thresh t
                                drop, slot);
 }
 
-// The same decision for rates of at most four planes (DEC_FEW): whole Philox calls and a mask per
-// kind of candidate.  With two planes there is little to share and lanes hardly differ:
-// (0.75,0.25) at 8192^2 in band passes takes 15.5 us per MCS this way, 16.3 with decide4.
+// The same decision for rates of at most three planes (DEC_FEW): whole Philox calls and a mask per
+// kind of candidate.  With so few planes there is little to share and lanes hardly differ.  A 4-MCS
+// band pass of 4096^2 at two CTAs per SM, this way against decide4: (0.75,0.25) 36.0 against 39.6
+// us, (0.875,0.125) 45.6 against 48.7, but (0.9375,0.0625), four planes, 55.1 against 46.8.  The
+// half-step kernel has its plane parts in a table and no instance of this: there decide4 is the
+// faster one from two planes on ((0.75,0.25) at 4096^2 13.6 us a MCS against 14.6).
 __device__ __forceinline__ uint4 decide4_few(uint4 cp, uint4 cq, Thresh tp, Thresh tq, Key key,
                                          uint32_t qgroup, uint32_t step, uint32_t stream)
 {
@@ -287,7 +290,7 @@ __device__ __forceinline__ uint4 decide4_few(uint4 cp, uint4 cq, Thresh tp, Thre
 //   DEC_NONE   no random plane can matter (every threshold is 0 or 2^32),
 //   DEC_ONE    at most the MSB plane matters (thresholds in {0, 2^31, 2^32}, e.g. p = 1/2),
 //   DEC_GENERAL anything else (bit-serial loop of decide4).
-//   DEC_FEW    DEC_GENERAL's rates of at most four planes, where a kernel has an instance of its own
+//   DEC_FEW    DEC_GENERAL's rates of at most three planes, where a kernel has an instance of its own
 //              for them (decide4_few).
 // And for kernels whose rates are known only at run time, as in a batch:
 //   DEC_ANY      any of these modes,
@@ -298,6 +301,14 @@ __host__ __device__ inline int dec_mode(Thresh tp, Thresh tq)
 {
     const int m = tp.planes > tq.planes ? tp.planes : tq.planes;
     return m == 0 ? DEC_NONE : m == 1 ? DEC_ONE : DEC_GENERAL;
+}
+
+// The same with DEC_FEW told apart.
+constexpr int DEC_FEW_PLANES = 3;
+__host__ __device__ inline int dec_mode_few(Thresh tp, Thresh tq)
+{
+    const int m = dec_mode(tp, tq);
+    return m == DEC_GENERAL && tp.planes <= DEC_FEW_PLANES && tq.planes <= DEC_FEW_PLANES ? (int)DEC_FEW : m;
 }
 
 // decide4 with the cheap modes spelled out; identical results in every mode.

@@ -342,7 +342,7 @@ cudaError_t scabit_fused(const uint32_t* d_src, uint32_t* d_dst, int lx, int ly,
 {
     const Key key = make_key(seed);
     const Thresh tp = make_thresh(Tp), tq = make_thresh(Tq);
-    const int mode = dec_mode(tp, tq);
+    const int mode = dec_mode_few(tp, tq);
     const bool useq = tq.always || tq.planes > 0;
 #define KPZB_FUSED_CASE(M)                                                                                    \
     return useq ? launch_fused_c<M, true>(d_src, d_dst, lx, ly, t0, key, stream_id, tp, tq, sh, d_counters,   \
@@ -351,7 +351,7 @@ cudaError_t scabit_fused(const uint32_t* d_src, uint32_t* d_dst, int lx, int ly,
                                            d_err, st)
     if (mode == DEC_NONE) KPZB_FUSED_CASE(DEC_NONE);
     if (mode == DEC_ONE) KPZB_FUSED_CASE(DEC_ONE);
-    if (tp.planes <= 4 && tq.planes <= 4) KPZB_FUSED_CASE(DEC_FEW);
+    if (mode == DEC_FEW) KPZB_FUSED_CASE(DEC_FEW);
     KPZB_FUSED_CASE(DEC_GENERAL);
 #undef KPZB_FUSED_CASE
 }

@@ -272,8 +272,7 @@ __device__ bool scabit_band(uint32_t* smem, const BandCtl& ctl, const BandGeom& 
     // that passes the x-carry by shuffles removed the atomics and bank conflicts but issued
     // 67 % more instructions and ran 15 % slower at 16384^2; the atomics stay.)
     __shared__ uint8_t slot_s[NT / 32][16];
-    const bool few = g.tp.planes <= 4 && g.tq.planes <= 4;
-    const int mode_rt = MODE < 0 ? (dec_mode(g.tp, g.tq) == DEC_GENERAL && few ? DEC_FEW : dec_mode(g.tp, g.tq)) : MODE;
+    const int mode_rt = MODE < 0 ? dec_mode_few(g.tp, g.tq) : MODE;
     const uint32_t wr = (uint32_t)Wr;
     const int gi = (G >= NT) ? (int)threadIdx.x : (int)(threadIdx.x & (G - 1));
     const int rstride = (G >= NT) ? 1 : NT >> lgG;

@@ -1,5 +1,5 @@
 """Batch passes with fewer work items than CTAs, as many, and more, at every number of CTAs per SM,
-in batches without and with rates of more than four random planes: every replica equals the
+in batches without and with rates that need the general decision: every replica equals the
 oracle.  The deepest pass that a lattice row fits in a CTA's shared memory, and the one beyond it."""
 import numpy as np
 import pytest
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("lxs,general", [([8], False), ([8] * 5, True), ([12], False), ([11, 12, 8], True),
                                          ([8] * 460, False), ([8] * 460, True)])
 def test_items_and_modes(kpzb, oracle, lxs, general, cps):
-    rates = [(1.0, 0.0), (0.5, 0.5), (0.75, 0.25), (0.9375, 0.0)] + ([(0.95, 0.05), (0.75, 0.1)] if general else [])
+    rates = [(1.0, 0.0), (0.5, 0.5), (0.75, 0.25), (0.875, 0.0)] + ([(0.95, 0.05), (0.75, 0.1), (0.9375, 0.0)] if general else [])
     pq = [rates[(i + len(lxs)) % len(rates)] for i in range(len(lxs))]
     b = kpzb.Batch(lxs, [r[0] for r in pq], [r[1] for r in pq], [40 + i for i in range(len(lxs))])
     b.setFusion(3, 2)
