@@ -757,7 +757,7 @@ def run_dt(args, world, rank, local):
     peak = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()).get("hbm_gbs", 6650.0) if (
         ROOT / "MEASURED_PEAKS.json").exists() else 6650.0
     ach = alg_launch / (per_launch * 1e-3) / 1e9
-    # DRAM bytes of one DT launch from an ncu capture of dt_kernel at 32768^2 (103.8 MB read +
+    # DRAM bytes of one DT launch from an ncu capture of the quadrant kernel at 32768^2 (103.8 MB read +
     # 36.3 MB written for 2^28 attempts), scaled by the lattice's sites: every launch reads and
     # writes its domain set's blocks and halos once, so the traffic grows with N
     traffic = round(DT_NCU_BYTES_32768 * N / (1 << 30)) if (not db4 and args.dt_inner == "dt") else None
@@ -781,7 +781,9 @@ def run_dt(args, world, rank, local):
                                f"flat start, p=0.95 q=0.05, random origin + shuffled domain sets per MCS, "
                                f"inner scheme {inner.upper()}"),
                   "mcs_per_step": m, "lattice": f"{1 << lx}x{1 << lx}", "parallelism": f"replicas x{world}"},
-                 roofline={"bound": "int-alu", "kernel": "dt_kernel", "achieved": int_roofline["achieved"],
+                 roofline={"bound": "int-alu",
+                           "kernel": "dt_quadrant_kernel" if db4 or args.dt_inner == "dt" else "dt_scatter_kernel",
+                           "achieved": int_roofline["achieved"],
                            "peak": int_roofline["peak"], "unit": "Tops/s (algorithmic integer ops)",
                            "frac": int_roofline["frac"], "traffic": traffic,
                            "peak_source": int_roofline["peak_source"] + "; of measured",
@@ -1093,13 +1095,13 @@ def run_gram(args, world, rank, local):
     g.close()
     s.close()
     return _line(tops, dt0 * 1e3, args, world,
-                 {"workload": "64x64 exact height Gram, 16384^2 lattice, slope snapshots, limbs built in shared "
-                              "memory, 3 int8 limbs, tcgen05 kind::i8",
+                 {"workload": "64x64 exact height Gram, 16384^2 lattice, slope snapshots, heights built in shared "
+                              "memory as one int8 limb (all within 126 of their mean), tcgen05 kind::i8",
                   "snapshots": 64, "sites": N},
                  unit="TOPS (2*64*64*N height-product ops / s)", dtype="int8->int32->int64",
                  int64_cuda_core_s=round(dt1, 4),
                  speedup_vs_int64=round(dt1 / dt0, 2), exact_match_int64=exact,
-                 roofline={"bound": "tensor", "kernel": "gram_tc_kernel", "achieved": round(tops, 1),
+                 roofline={"bound": "tensor", "kernel": "gram_low_kernel", "achieved": round(tops, 1),
                            "peak": round(int8_peak, 1),
                            "unit": "TOPS (the Gram's 2*64*64*N algorithmic ops against the int8 tcgen05 peak)",
                            "frac": round(tops / int8_peak, 4), "traffic": None,

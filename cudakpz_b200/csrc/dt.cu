@@ -859,7 +859,7 @@ kpzb_status dt_enqueue(DtState* s, uint32_t* d_local, int lx, int ly, uint64_t t
             for (int a = 0; a < 4; ++a) launch(ox, oy, order[a], t);
         }
         const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_fail(e, "dt_kernel");
+        if (e != cudaSuccess) return cuda_fail(e, "DT launch");
     }
     return KPZB_OK;
 }
