@@ -406,8 +406,8 @@ static void mark_wait(kpzb_handle* h)
 }
 
 // Whether the left-over MCS of a call may go through the second buffer: not while the caller
-// captures the stream (nothing may be allocated, and a graph of less than one pass keeps
-// updating the lattice in place), nor when there is no memory for it.
+// captures the stream (a graph of less than one pass keeps updating the lattice in place), nor,
+// where no pass of the plan's depth fits and has asked for the buffer already, without memory for it.
 static bool spare_buffer(kpzb_handle* h)
 {
     if (capturing(h)) return false;
@@ -442,7 +442,7 @@ static kpzb_status enqueue_sca(kpzb_handle* h, int n)
             done += k;
         }
     } else if (k > 1 && plan.kind == PASS_WAVE && ws.ok) {
-        mark_wait(h);
+        if (n >= k) mark_wait(h);
         kpzb_status s = ensure_tmp(h);
         if (s != KPZB_OK) return s;
         while (n - done >= k) {
@@ -456,7 +456,7 @@ static kpzb_status enqueue_sca(kpzb_handle* h, int n)
     } else if (k > 1 && plan.kind == PASS_STREAM) {
         const StreamShape ss = scabit_stream_shape(h->lx, h->ly, k, h->sm_count, plan.cps ? plan.cps : 1);
         if (ss.ok) {
-            mark_wait(h);
+            if (n >= k) mark_wait(h);
             kpzb_status s = ensure_tmp(h);
             if (s != KPZB_OK) return s;
             while (n - done >= k) {
@@ -471,7 +471,7 @@ static kpzb_status enqueue_sca(kpzb_handle* h, int n)
     } else if (k > 1) {
         FusedShape fs = scabit_fused_shape_cps(h->lx, h->ly, k, plan.cps, 0);
         if (fs.ok) {
-            mark_wait(h);
+            if (n >= k) mark_wait(h);
             kpzb_status s = ensure_tmp(h);
             if (s != KPZB_OK) return s;
             while (n - done >= k) {
@@ -488,8 +488,9 @@ static kpzb_status enqueue_sca(kpzb_handle* h, int n)
     // tiles of about the same height, or of the band kernel, which takes any depth.  One pass of r
     // MCS reads and writes the lattice once where 2r half-step launches do so 2r times: 50 MCS of
     // 16384^2 at (1,0) end in 27 us instead of 71, 10 MCS of 256^2 in two launches instead of seven.
-    // A lone last MCS of the warp-tile kernel's lattices stays two half-steps.
-    const bool spare = k > 1 && done < n && spare_buffer(h);
+    // A lone last MCS of the warp-tile kernel's lattices stays two half-steps, and so do the left-over
+    // MCS of the streaming and the full-width register kernel.
+    const bool spare = k > 1 && done < n && (plan.kind == PASS_STRIP || plan.kind == PASS_BAND) && spare_buffer(h);
     if (spare && plan.kind == PASS_STRIP) {
         for (int r = 6; r >= 2; r -= 2) {
             const int cycle = strip_cycle_rows(r);
