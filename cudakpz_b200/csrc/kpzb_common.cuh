@@ -311,7 +311,28 @@ __host__ __device__ inline int dec_mode_few(Thresh tp, Thresh tq)
     return m == DEC_GENERAL && tp.planes <= DEC_FEW_PLANES && tq.planes <= DEC_FEW_PLANES ? (int)DEC_FEW : m;
 }
 
-// decide4 with the cheap modes spelled out; identical results in every mode.
+// decide4 for at most one random plane (DEC_NONE, DEC_ONE); identical results.
+__device__ __forceinline__ uint4 decide4_one(int mode, uint4 cp, uint4 cq, Thresh tp, Thresh tq, Key key,
+                                             uint32_t qgroup, uint32_t step, uint32_t stream)
+{
+    if (mode == DEC_NONE) {
+        const uint32_t ap = tp.always ? 0xFFFFFFFFu : 0u, aq = tq.always ? 0xFFFFFFFFu : 0u;
+        return make_uint4((cp.x & ap) | (cq.x & aq), (cp.y & ap) | (cq.y & aq),
+                          (cp.z & ap) | (cq.z & aq), (cp.w & ap) | (cq.w & aq));
+    }
+    // a threshold with one plane is 2^31: sites whose MSB of u is 0 flip
+    const uint32_t any = cp.x | cp.y | cp.z | cp.w | cq.x | cq.y | cq.z | cq.w;
+    uint4 r = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+    if (any) r = philox4x32_10(make_uint4(qgroup, step, TAG_SCA << 8, stream), key);
+    const uint32_t ap = tp.always ? 0xFFFFFFFFu : 0u, aq = tq.always ? 0xFFFFFFFFu : 0u;
+    const uint32_t hp = tp.planes ? 0xFFFFFFFFu : 0u, hq = tq.planes ? 0xFFFFFFFFu : 0u;
+    return make_uint4((cp.x & (ap | (hp & ~r.x))) | (cq.x & (aq | (hq & ~r.x))),
+                      (cp.y & (ap | (hp & ~r.y))) | (cq.y & (aq | (hq & ~r.y))),
+                      (cp.z & (ap | (hp & ~r.z))) | (cq.z & (aq | (hq & ~r.z))),
+                      (cp.w & (ap | (hp & ~r.w))) | (cq.w & (aq | (hq & ~r.w))));
+}
+
+// The decision in any mode.
 // slot: sixteen bytes of shared memory per warp where all 32 lanes call together, else nullptr.
 // GENERAL: false where DEC_GENERAL is not among the caller's modes.
 template <bool WARP = false, bool GENERAL = true>
@@ -319,23 +340,7 @@ __device__ __forceinline__ uint4 decide4_mode(int mode, uint4 cp, uint4 cq, Thre
                                               Key key, uint32_t qgroup, uint32_t step,
                                               uint32_t stream, uint8_t* slot = nullptr)
 {
-    if (mode == DEC_NONE) {
-        const uint32_t ap = tp.always ? 0xFFFFFFFFu : 0u, aq = tq.always ? 0xFFFFFFFFu : 0u;
-        return make_uint4((cp.x & ap) | (cq.x & aq), (cp.y & ap) | (cq.y & aq),
-                          (cp.z & ap) | (cq.z & aq), (cp.w & ap) | (cq.w & aq));
-    }
-    if (mode == DEC_ONE) {
-        // a threshold with one plane is 2^31: sites whose MSB of u is 0 flip
-        const uint32_t any = cp.x | cp.y | cp.z | cp.w | cq.x | cq.y | cq.z | cq.w;
-        uint4 r = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-        if (any) r = philox4x32_10(make_uint4(qgroup, step, TAG_SCA << 8, stream), key);
-        const uint32_t ap = tp.always ? 0xFFFFFFFFu : 0u, aq = tq.always ? 0xFFFFFFFFu : 0u;
-        const uint32_t hp = tp.planes ? 0xFFFFFFFFu : 0u, hq = tq.planes ? 0xFFFFFFFFu : 0u;
-        return make_uint4((cp.x & (ap | (hp & ~r.x))) | (cq.x & (aq | (hq & ~r.x))),
-                          (cp.y & (ap | (hp & ~r.y))) | (cq.y & (aq | (hq & ~r.y))),
-                          (cp.z & (ap | (hp & ~r.z))) | (cq.z & (aq | (hq & ~r.z))),
-                          (cp.w & (ap | (hp & ~r.w))) | (cq.w & (aq | (hq & ~r.w))));
-    }
+    if (mode == DEC_NONE || mode == DEC_ONE) return decide4_one(mode, cp, cq, tp, tq, key, qgroup, step, stream);
     if (!GENERAL || mode == DEC_FEW) return decide4_few(cp, cq, tp, tq, key, qgroup, step, stream);
     return decide4<WARP>(cp, cq, tp, tq, key, qgroup, PlaneMaker{step, key}, stream, slot);
 }

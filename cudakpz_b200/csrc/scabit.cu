@@ -41,11 +41,11 @@ scabit_half_kernel(uint32_t* __restrict__ sys, int lx, int ly, int sigma, uint32
 {
     __shared__ uint32_t nxt_s[SCABIT_THREADS];
     __shared__ uint32_t carry_s[2][SCABIT_THREADS];
-    __shared__ uint8_t slot_s[SCABIT_THREADS / 32][16];
+    __shared__ uint8_t slot_s[GENERAL ? SCABIT_THREADS / 32 : 1][16];
 
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int lin = ty * TX + tx;
-    [[maybe_unused]] uint8_t* slot = slot_s[lin >> 5];
+    [[maybe_unused]] uint8_t* slot = slot_s[GENERAL ? lin >> 5 : 0];
     const uint64_t Wr = 1ull << (lx - 6);
     const uint64_t Q = 1ull << (lx + ly - 6);
     const uint64_t rows = 1ull << ly;
@@ -102,8 +102,7 @@ scabit_half_kernel(uint32_t* __restrict__ sys, int lx, int ly, int sigma, uint32
             } else if constexpr (GENERAL) {
                 m = decide4<true>(cp, cq, tp, tq, key, (uint32_t)((roff + wi) >> 2), planes, stream, slot);
             } else {
-                m = decide4_mode(dec_mode(tp, tq), cp, cq, tp, tq, key, (uint32_t)((roff + wi) >> 2), step,
-                                 stream);
+                m = decide4_one(dec_mode(tp, tq), cp, cq, tp, tq, key, (uint32_t)((roff + wi) >> 2), step, stream);
             }
             if (COUNT) {
                 ndep += __popc(m.x & cp.x) + __popc(m.y & cp.y) + __popc(m.z & cp.z) + __popc(m.w & cp.w);
