@@ -61,3 +61,42 @@ def test_walk_matches_oracle(kpzb, oracle, kind, lx, ly):
     np.testing.assert_allclose([r.w2] + r.h, ref[:8], rtol=1e-12, atol=1e-12)
     np.testing.assert_allclose(ch, ref[8], rtol=1e-10, atol=1e-12 * max(1.0, abs(tag.h[0] * r.h[0])))
     assert cs == ref[9]
+
+
+def exact_sums(h, g):
+    """Whole-number sums of h^k, |h|^k (k = 1..7) and of h g over all sites."""
+    lo = int(h.min())
+    n = np.bincount((h - lo).ravel())
+    at = [(int(i) + lo, int(n[i])) for i in np.flatnonzero(n)]
+    cross = h.astype(np.int64).ravel() * g.astype(np.int64).ravel()
+    cross = (int((cross >> 20).sum()) << 20) + int((cross & ((1 << 20) - 1)).sum())
+    return [sum(c * x**k for x, c in at) for k in range(1, 8)], [sum(c * abs(x) ** k for x, c in at) for k in range(1, 8)], cross
+
+
+@pytest.mark.parametrize("kind", ["grown", "steep", "words"])
+@pytest.mark.parametrize("lx,ly", [(8, 13), (8, 17), (15, 4), (16, 3), (20, 3)])
+def test_tall_and_wide_lattices(kpzb, oracle, kind, lx, ly):
+    """Blocks of 32 and of 512 rows (several steps of a block's row loop), and rows whose quarters
+    take several steps of a warp, against whole-number sums of the oracle's heights: the oracle's own
+    sums in FP64 lose digits to heights of thousands that cancel.  The higher moments are off by at
+    most 1e-12 of their terms' size, the covariance by that of its two terms."""
+    N = 1 << (lx + ly)
+    w = surface(oracle, kind, lx, ly)
+    cur = w ^ np.where(np.arange(w.size) % 5 == 0, np.uint32(0x01020810), np.uint32(0))  # open rows
+    h, g = oracle.heights(w, lx, ly, oracle.ENC_CBBIT), oracle.heights(cur, lx, ly, oracle.ENC_CBBIT)
+    s = kpzb.Scheduler(lx, ly)
+    s.pushSystem(w)
+    sums, size, _ = exact_sums(h, h)
+    assert s.heightSums() == ((sums[0], sums[1]), (int(h.min()), int(h.max())))
+    tag = s.correlateTag()
+    for k in range(7):
+        assert abs(tag.h[k] - sums[k] / N) <= 1e-12 * size[k] / N, k
+    s.pushSystem(cur)
+    r, ch, cs = s.correlate()
+    s.close()
+    sums_g, size, cross = exact_sums(g, h)
+    for k in range(7):
+        assert abs(r.h[k] - sums_g[k] / N) <= 1e-12 * size[k] / N, k
+    exact = (cross * N - sums[0] * sums_g[0]) / N**2
+    assert abs(ch - exact) <= 1e-12 * (abs(cross) / N + abs(sums[0] * sums_g[0]) / N**2)
+    assert cs == oracle.correlate(cur, w, lx, ly, oracle.ENC_CBBIT, tag.h[0])[9]
