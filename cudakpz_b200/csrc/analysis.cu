@@ -259,11 +259,11 @@ __device__ __forceinline__ long long row_block_bases(const RowBlock* blocks, int
 // A group of eight sites is its height H before the first site and an 8-bit slope pattern, so
 // the sums of h^k over the lattice follow from counts of (H, pattern) alone.  Each CTA keeps the
 // counts of WALK_BINS heights of one parity x 256 patterns in shared memory and adds one per
-// group: a shared atomic and about ten integer instructions for eight sites, where evaluating
-// the powers site by site took about 17 instructions a site (330 us against 49 us at 2^28 sites,
-// where the integer ALU bound it; now the shared atomics do; 70 against 25 us at 2^26).  The even rows' groups all have
-// heights of one parity and the odd rows' of the other, so a CTA walks rows of one parity and
-// a bin covers two heights.  At the end thread (pattern p, slice of heights) takes the power
+// group: 27 instructions for eight sites, one of them a shared atomic, where evaluating the powers
+// site by site took about 17 a site (330 us against 49 us at 2^28 sites, 70 against 25 at 2^26).  The
+// integer ALU bounds it (76 % active at 2^30 sites; the atomics, 4.8 wavefronts each, keep shared
+// memory half busy).  The even rows' groups all have heights of one parity and the odd rows' of the
+// other, so a CTA walks rows of one parity and a bin covers two heights.  At the end thread (pattern p, slice of heights) takes the power
 // sums of H over its bins and combines them with the pattern's own offsets' power sums.
 //
 // Counts are exact and the bins' heights span less than 2^9, so every term up to k = 7 of a

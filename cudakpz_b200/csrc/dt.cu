@@ -260,8 +260,9 @@ __device__ __forceinline__ uint32_t not_adjacent(uint32_t pos, uint32_t right, u
 // kpz/kpzSimulationPrimitivesTemplates_BaseInnerDB.cu:110-163).  Two attempts of a round touch a
 // common bit only if one's site is the other's right or lower neighbour, and then the former
 // lies in an earlier phase.  All attempts without such a neighbour commute, so they are done in
-// one pass; the others (0.34 % of all, known from the positions alone) follow in their phases'
-// order.  That takes one attempt's instructions and 1.8 barriers per round instead of 2.4 and 3.
+// one pass; the others (0.39 % of all, known from the positions alone) follow in their phases'
+// order.  That takes one pass and on average 2.1 barriers a round (a block of 512 cells has two such
+// attempts a round) instead of three of each.
 // Columns, rows and word offsets of four rounds are formed as bytes of one word.  Measured on a
 // B200, DBSH at p = 0.95, q = 0.05: 16384^2 1592 -> 1248 us per MCS, 1024^2 181 -> 156 us (a launch
 // there is 8 blocks, 64 rounds one after the other); DBSHRep 1583 -> 1239, DTDBSH 929 -> 779 us at
@@ -543,7 +544,7 @@ dt_scatter_kernel(uint32_t* __restrict__ sys, int lxw, int lyw, int lnbx, int ox
 // 32 x 16 threads, one cell each, on the block's ENC_LOCAL words in shared memory (65 x 33 with the
 // halo).  No two sites of a round share a word, so a round needs one barrier and its flips only
 // order themselves.  A per-launch table of 8-byte entries turns (quadrant, position) into the three
-// words' byte offsets and three rotate amounts.  67 instructions an attempt, most of them on the
+// words' byte offsets and three rotate amounts.  59 instructions an attempt, most of them on the
 // integer ALU (2 cycles each per warp and scheduler), which bounds it.  Holding the cells in
 // registers instead (quadrant and neighbours by shifts and shuffles, no tile and no barrier in most
 // rounds) took 63 and was 2 % faster at 16384^2 and 10 % slower below 4096^2, and was dropped.

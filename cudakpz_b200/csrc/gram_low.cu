@@ -1,13 +1,13 @@
 // gram_low.cu -- exact Gram of snapshots whose shifted heights fit one int8 limb (sm_100a).
 //
 // The snapshots' height ranges are known from when they were added; where every v = h - c lies in
-// [-126, 126] (a row's b(y), at most one beyond, then also fits a byte), v is its own int8 operand and no tile ever needs the three-limb form of
-// gram_tc.cu.  That removes the need to hand tiles of two kinds to one issuing thread, which is
+// [-126, 126] (a row's b(y), at most one beyond, then also fits a byte), v is its own int8 operand and
+// no tile ever needs the three-limb form of gram_tc.cu.  That removes the need to hand tiles of two kinds to one issuing thread, which is
 // what bounded that kernel: at 16384^2 its barrier round trip between eight producers and one
 // consumer took 4.5 of its 9.0 ms with nothing built, loaded or multiplied.  Measured on a B200, 64
 // snapshots: 16384^2 9.05 -> 3.07 ms, 4096^2 0.76 -> 0.31 ms; what bounds it now is shared memory
-// (lookups, row stores and 6 KB of MMA operands per K step) and the integer ALU (about ten
-// operations per eight sites), about equally.
+// (lookups, row stores and 6 KB of MMA operands per K step: 68 % of its wavefronts at 8192^2) and the
+// integer ALU (24 instructions for eight sites of a snapshot, 59 % active).
 //
 // Here sixteen warps form eight pairs, and a pair does everything for its own contiguous run of
 // 128-site tiles (gram_slope.cuh gives the walk): lane l of its two warps walks snapshots l and
@@ -23,7 +23,7 @@
 // Four sites per table lookup: the 4-bit pattern of two even and two odd X-slope bits gives the
 // four cumulative steps as bytes (biased by 4), added to the broadcast value before them; sixteen
 // 4-byte entries lie in sixteen banks, so a warp's lookups never conflict (a 256-entry table of
-// eight steps took 4.5 wavefronts a lookup).
+// eight steps takes about five wavefronts a lookup).
 //
 // Sums: |v v'| <= r^2 for the largest |v| = r, so an int32 accumulator holds `window` tiles, after
 // which (and at the end) the pair's warps add its 64 x 64 block to the int64 result.
