@@ -30,22 +30,23 @@ constexpr int SCABIT_THREADS = 256;
 // bit 0 in the X quadrants, bit 1 in the Y quadrants, i.e. the ENC_LOCAL class words put
 // through the lattice codec), dr the four classes' thresholds (Disorder2SyncRng,
 // kpz/kpzSCACores.cu:217-280).
-// GENERAL: rates of more than one random plane (and disorder); their plane parts come as a table.
+// MODE: DEC_NONE, DEC_ONE, or DEC_GENERAL for rates of more random planes and disorder, whose plane
+// parts come as a table.
 struct NoPlanes {};
-template <bool COUNT, bool DIS, bool GENERAL>
+template <bool COUNT, bool DIS, int MODE>
 __global__ void __launch_bounds__(SCABIT_THREADS)
 scabit_half_kernel(uint32_t* __restrict__ sys, int lx, int ly, int sigma, uint32_t step, Key key,
                    uint32_t stream, Thresh tp, Thresh tq, int TX, int TY,
                    unsigned long long* __restrict__ counters, const uint32_t* __restrict__ dis,
-                   DisorderRates dr, const std::conditional_t<GENERAL, PlaneTable, NoPlanes> planes)
+                   DisorderRates dr, const std::conditional_t<MODE == DEC_GENERAL, PlaneTable, NoPlanes> planes)
 {
     __shared__ uint32_t nxt_s[SCABIT_THREADS];
     __shared__ uint32_t carry_s[2][SCABIT_THREADS];
-    __shared__ uint8_t slot_s[GENERAL ? SCABIT_THREADS / 32 : 1][16];
+    __shared__ uint8_t slot_s[MODE == DEC_GENERAL ? SCABIT_THREADS / 32 : 1][16];
 
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int lin = ty * TX + tx;
-    [[maybe_unused]] uint8_t* slot = slot_s[GENERAL ? lin >> 5 : 0];
+    [[maybe_unused]] uint8_t* slot = slot_s[MODE == DEC_GENERAL ? lin >> 5 : 0];
     const uint64_t Wr = 1ull << (lx - 6);
     const uint64_t Q = 1ull << (lx + ly - 6);
     const uint64_t rows = 1ull << ly;
@@ -99,10 +100,10 @@ scabit_half_kernel(uint32_t* __restrict__ sys, int lx, int ly, int sigma, uint32
                 const uint4 d0 = *reinterpret_cast<const uint4*>(dis + bthisX + roff + wi);
                 const uint4 d1 = *reinterpret_cast<const uint4*>(dis + bthisY + roff + wi);
                 m = decide4_dis(cp, cq, d0, d1, dr, key, (uint32_t)((roff + wi) >> 2), planes, stream, slot);
-            } else if constexpr (GENERAL) {
+            } else if constexpr (MODE == DEC_GENERAL) {
                 m = decide4<true>(cp, cq, tp, tq, key, (uint32_t)((roff + wi) >> 2), planes, stream, slot);
             } else {
-                m = decide4_one(dec_mode(tp, tq), cp, cq, tp, tq, key, (uint32_t)((roff + wi) >> 2), step, stream);
+                m = decide4_one(MODE, cp, cq, tp, tq, key, (uint32_t)((roff + wi) >> 2), step, stream);
             }
             if (COUNT) {
                 ndep += __popc(m.x & cp.x) + __popc(m.y & cp.y) + __popc(m.z & cp.z) + __popc(m.w & cp.w);
@@ -177,13 +178,18 @@ cudaError_t scabit_half(uint32_t* d_sys, int lx, int ly, int sigma, uint32_t ste
                                         nullptr, dr, planes);
         return cudaGetLastError();
     };
-    if (dec_mode(tp, tq) == DEC_GENERAL) {
+    switch (dec_mode(tp, tq)) {
+    case DEC_NONE:
+        return d_counters ? go(scabit_half_kernel<true, false, DEC_NONE>, NoPlanes{})
+                          : go(scabit_half_kernel<false, false, DEC_NONE>, NoPlanes{});
+    case DEC_ONE:
+        return d_counters ? go(scabit_half_kernel<true, false, DEC_ONE>, NoPlanes{})
+                          : go(scabit_half_kernel<false, false, DEC_ONE>, NoPlanes{});
+    default:
         const PlaneTable planes = make_plane_table(step, key);
-        return d_counters ? go(scabit_half_kernel<true, false, true>, planes)
-                          : go(scabit_half_kernel<false, false, true>, planes);
+        return d_counters ? go(scabit_half_kernel<true, false, DEC_GENERAL>, planes)
+                          : go(scabit_half_kernel<false, false, DEC_GENERAL>, planes);
     }
-    return d_counters ? go(scabit_half_kernel<true, false, false>, NoPlanes{})
-                      : go(scabit_half_kernel<false, false, false>, NoPlanes{});
 }
 
 cudaError_t scabit_half_dis(uint32_t* d_sys, const uint32_t* d_dis_cbbit, int lx, int ly, int sigma,
@@ -195,7 +201,7 @@ cudaError_t scabit_half_dis(uint32_t* d_sys, const uint32_t* d_dis_cbbit, int lx
     const DisorderRates dr = make_disorder_rates(Tp, Tq);
     const PlaneTable planes = make_plane_table(step, key);
     dim3 block(sh.TX, sh.TY);
-    auto kern = d_counters ? scabit_half_kernel<true, true, true> : scabit_half_kernel<false, true, true>;
+    auto kern = d_counters ? scabit_half_kernel<true, true, DEC_GENERAL> : scabit_half_kernel<false, true, DEC_GENERAL>;
     kern<<<sh.grid, block, 0, st>>>(d_sys, lx, ly, sigma, step, key, stream_id, dr.tp[0], dr.tq[0], sh.TX, sh.TY,
                                     d_counters, d_dis_cbbit, dr, planes);
     return cudaGetLastError();
