@@ -263,8 +263,9 @@ __device__ __forceinline__ long long row_block_bases(const RowBlock* blocks, int
 // site by site took about 17 a site (330 us against 49 us at 2^28 sites, 70 against 25 at 2^26).  The
 // integer ALU bounds it (76 % active at 2^30 sites; the atomics, 4.8 wavefronts each, keep shared
 // memory half busy).  The even rows' groups all have heights of one parity and the odd rows' of the
-// other, so a CTA walks rows of one parity and a bin covers two heights.  At the end thread (pattern p, slice of heights) takes the power
-// sums of H over its bins and combines them with the pattern's own offsets' power sums.
+// other, so a CTA walks rows of one parity and a bin covers two heights.  At the end thread (pattern
+// p, slice of heights) takes the power sums of H over its bins and combines them with the pattern's
+// own offsets' power sums.
 //
 // Counts are exact and the bins' heights span less than 2^9, so every term up to k = 7 of a
 // surface with |H| <= 16 is an exact integer in FP64; above that the terms of one bin do not
